@@ -371,9 +371,10 @@ int jg_destroy(jg_case_t* h) {
 // Greedy colouring of the cell graph (neighbours through internal faces) in cell order: each cell
 // takes the smallest colour none of its lower-numbered neighbours has.  With at most
 // MAX_COLOR_LISTS colours, also the slices holding a cell of each colour, colour by colour
-// (cslices[coff[q] .. coff[q+1])).  Returns the number of colours.
+// (cslices[coff[q] .. coff[q+1])).  Returns the number of colours.  proper: no cell is coupled to one
+// of its own colour (false where a face joins a cell to itself or the colours ran out).
 static int color_cells(const jg_mesh* mesh, std::vector<uint8_t>& color, std::vector<int>& cslices,
-                       std::vector<int>& coff) {
+                       std::vector<int>& coff, bool* proper = nullptr) {
   const int N = mesh->ncv;
   std::vector<int> adj_i(N + 1, 0), adj_v;
   for (int f = mesh->nfa_b; f < mesh->nfa; f++) {
@@ -386,6 +387,7 @@ static int color_cells(const jg_mesh* mesh, std::vector<uint8_t>& color, std::ve
     std::vector<int> fill(adj_i.begin(), adj_i.end() - 1);
     for (int f = mesh->nfa_b; f < mesh->nfa; f++) {
       const int a = mesh->cvofa[2 * f], b = mesh->cvofa[2 * f + 1];
+      if (proper && a == b) *proper = false;
       adj_v[fill[a]++] = b;
       adj_v[fill[b]++] = a;
     }
@@ -399,6 +401,7 @@ static int color_cells(const jg_mesh* mesh, std::vector<uint8_t>& color, std::ve
     int k = 0;
     while (k < 255 && mark[k] == c) k++;
     color[c] = (uint8_t)k;
+    if (proper && k == 255) *proper = false;
     ncolors = std::max(ncolors, k + 1);
   }
   cslices.clear();
@@ -490,6 +493,38 @@ static int build(jg_case* h, const jg_mesh* mesh, const jg_params* q) {
     bf_i[c + 1] = (int)bf_v.size();
     h->cell_cols[c + 1] = (int)h->col_nb.size();
   }
+  // LINE relaxation: a line cell's columns are its couplings off the line first, then those to its
+  // line neighbours (each group in face order), so that the sweeps' pass over the off-line couplings
+  // reads the front columns of a slice only.  noff: off-line columns of each cell
+  std::vector<int> line_off, line_cv, line_prev, line_next;
+  std::vector<int> noff;
+  if (q->lin_solver == JG_LS_BCGSTAB_LINELET || q->lin_solver == JG_LS_LINE)
+    multi_cell_lines(mesh, h->rn.face_old, line_off, line_cv, q->lin_solver == JG_LS_LINE);
+  if (q->lin_solver == JG_LS_LINE) {
+    noff = ncols;
+    line_prev.assign(N, -1);
+    line_next.assign(N, -1);
+    for (size_t l = 0; l + 1 < line_off.size(); l++)
+      for (int k = line_off[l]; k < line_off[l + 1]; k++) {
+        if (k > line_off[l]) line_prev[line_cv[k]] = line_cv[k - 1];
+        if (k + 1 < line_off[l + 1]) line_next[line_cv[k]] = line_cv[k + 1];
+      }
+    std::vector<int> col_new, nbs;
+    for (int c = 0; c < N; c++) {
+      int* nbv = h->col_nb.data() + h->cell_cols[c];
+      auto inl = [&](int j) { return nbv[j] == line_prev[c] || nbv[j] == line_next[c]; };
+      int off = 0;
+      for (int j = 0; j < ncols[c]; j++) off += !inl(j);
+      noff[c] = off;
+      if (off == ncols[c]) continue;
+      col_new.assign(ncols[c], 0);
+      nbs.assign(nbv, nbv + ncols[c]);
+      for (int j = 0, a = 0, b = off; j < ncols[c]; j++) col_new[j] = inl(j) ? b++ : a++;
+      for (int j = 0; j < ncols[c]; j++) nbv[col_new[j]] = nbs[j];
+      for (int k = fi[c]; k < fi[c + 1]; k++)
+        if (slots[k].col >= 0) slots[k].col = col_new[slots[k].col];
+    }
+  }
   // sliced ELL
   int nslices = (N + SLICE - 1) / SLICE;
   h->ell_off.assign(nslices + 1, 0);
@@ -520,7 +555,8 @@ static int build(jg_case* h, const jg_mesh* mesh, const jg_params* q) {
   // colour the slices that hold a cell of that colour (a colour pass launches over these only)
   std::vector<uint8_t> color;
   std::vector<int> cslices, coff;
-  const int ncolors = color_cells(mesh, color, cslices, coff);
+  bool proper = true;
+  const int ncolors = color_cells(mesh, color, cslices, coff, &proper);
   h->ncolors = ncolors;
   // device mesh
   Mesh& m = h->m;
@@ -557,6 +593,7 @@ static int build(jg_case* h, const jg_mesh* mesh, const jg_params* q) {
   RC(upload(h, &m.ell_lower, ell_lower.data(), ell_lower.size()));
   RC(upload(h, &m.color, color.data(), color.size()));
   m.ncolors = ncolors;
+  m.color_proper = proper;
   launch_face_geo(m, (double*)m.fa_u, (double*)m.fa_s, h->stream);
   CKL();
   // device state
@@ -691,8 +728,7 @@ static int build(jg_case* h, const jg_mesh* mesh, const jg_params* q) {
     CKL();
   }
   if (q->lin_solver == JG_LS_BCGSTAB_LINELET || q->lin_solver == JG_LS_LINE) {
-    std::vector<int> off, cv;
-    multi_cell_lines(mesh, h->rn.face_old, off, cv, q->lin_solver == JG_LS_LINE);
+    std::vector<int>&off = line_off, &cv = line_cv;
     Lines& L = h->lines;
     L.nlines = (int)off.size() - 1;
     const size_t nc = std::max<size_t>(cv.size(), 1);
@@ -725,25 +761,19 @@ static int build(jg_case* h, const jg_mesh* mesh, const jg_params* q) {
       RC(dmalloc(h, &L.up, 25 * nc));
       RC(dmalloc(h, &L.v, 5 * nc));
     } else {
-      // the line cells and, per ELL entry, whether it couples a cell to its predecessor or successor on its line
-      std::vector<uint8_t> on_line(N, 0), inl((size_t)rows * SLICE, 0);
-      std::vector<int> prev(N, -1), next(N, -1);
-      for (int l = 0; l < L.nlines; l++)
-        for (int k = off[l]; k < off[l + 1]; k++) {
-          on_line[cv[k]] = 1;
-          if (k > off[l]) prev[cv[k]] = cv[k - 1];
-          if (k + 1 < off[l + 1]) next[cv[k]] = cv[k + 1];
-        }
-      for (int c = 0; c < N; c++) {
-        if (!on_line[c]) continue;
-        const int sl = c / SLICE, lane = c % SLICE;
-        for (int j = 0; j < ncols[c]; j++) {
-          const size_t e = (size_t)(h->ell_off[sl] + j) * SLICE + lane;
-          if (ell_nb[e] == prev[c] || ell_nb[e] == next[c]) inl[e] = 1;
-        }
+      // the line cells, and per cell the ELL rows of its couplings off the line and per slice their end
+      std::vector<uint8_t> on_line(N, 0);
+      std::vector<int> off_end(nslices);
+      for (int k = 0; k < L.nlines; k++)
+        for (int i = off[k]; i < off[k + 1]; i++) on_line[cv[i]] = 1;
+      for (int sl = 0; sl < nslices; sl++) {
+        int w = 0;
+        for (int c = sl * SLICE; c < std::min(N, (sl + 1) * SLICE); c++) w = std::max(w, noff[c]);
+        off_end[sl] = h->ell_off[sl] + w;
       }
       RC(upload(h, &L.on_line, on_line.data(), on_line.size()));
-      RC(upload(h, &L.ell_inline, inl.data(), inl.size()));
+      RC(upload(h, &L.noff, noff.data(), noff.size()));
+      RC(upload(h, &L.off_end, off_end.data(), off_end.size()));
       RC(dmalloc_bytes(h, &L.binv, (size_t)bs * bs * nc * h->eltsz));
       RC(dmalloc_bytes(h, &L.blow, (size_t)bs * bs * nc * h->eltsz));
       RC(dmalloc_bytes(h, &L.bup, (size_t)bs * bs * nc * h->eltsz));
@@ -863,7 +893,8 @@ static size_t footprint(const jg_mesh* mesh, const jg_params* q, const std::vect
     if (q->lin_solver == JG_LS_BCGSTAB_LINELET)
       b += 3 * alloc_round(25 * nc * d) + alloc_round(5 * nc * d);
     else
-      b += alloc_round(N) + alloc_round(rows * SLICE) + 3 * alloc_round(b2 * nc * e) + alloc_round(bs * nc * e);
+      b += alloc_round(N) + alloc_round(N * i) + alloc_round(nslices * i) + 3 * alloc_round(b2 * nc * e) +
+           alloc_round(bs * nc * e);
   }
   return b;
 }

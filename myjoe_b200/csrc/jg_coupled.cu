@@ -18,6 +18,7 @@
 #include "jg_cell.cuh"
 #include "jg_flux.cuh"
 #include "jg_internal.h"
+#include "jg_sweep.cuh"
 
 namespace jg {
 
@@ -1162,71 +1163,6 @@ __global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb
   }
 }
 
-// ---------------------------------------------------------------------------
-// block relaxation of the B x B system: one warp per block row of a 32-cell
-// slice (B*32 threads), as the 5x5 sweeps
-// ---------------------------------------------------------------------------
-template <typename BT, int B>
-__global__ void __launch_bounds__(B * 32) k_jacobi_c(Mesh m, State st, const BT* __restrict__ xin,
-                                                      BT* __restrict__ xout, int first) {
-  __shared__ BT sacc[B][SLICE];
-  const int row = threadIdx.x / SLICE, lane = threadIdx.x % SLICE;
-  const int slice = blockIdx.x;
-  const int c = slice * SLICE + lane;
-  const bool active = c < m.ncv && st.case_active[m.case_of[c]];
-  const int N = m.ncv;
-  BT acc = active ? (BT)st.b[(size_t)B * c + row] : (BT)0;
-  if (!first && active) {
-    const BT* O = (const BT*)st.O;
-    for (int j = m.ell_off[slice]; j < m.ell_off[slice + 1]; j++) {
-      int nb = m.ell_nb[(size_t)j * SLICE + lane];
-      const BT* Ob = O + ((size_t)j * B * B + B * row) * SLICE + lane;
-      BT s = 0;
-      for (int k = 0; k < B; k++) s += Ob[k * SLICE] * xin[(size_t)k * N + nb];
-      acc -= s;
-    }
-  }
-  sacc[row][lane] = acc;
-  __syncthreads();
-  if (active) {
-    const BT* Di = (const BT*)st.Dinv;
-    BT s = 0;
-    for (int k = 0; k < B; k++) s += Di[(size_t)(B * row + k) * N + c] * sacc[k][lane];
-    xout[(size_t)row * N + c] = s;
-  }
-}
-
-template <typename BT, int B>
-__global__ void __launch_bounds__(B * 32) k_gs_c(Mesh m, State st, BT* __restrict__ x, int color,
-                                                 const int* __restrict__ slices) {
-  __shared__ BT sacc[B][SLICE];
-  const int row = threadIdx.x / SLICE, lane = threadIdx.x % SLICE;
-  const int slice = slices ? slices[blockIdx.x] : blockIdx.x;  // slices: those holding this colour
-  const int c = slice * SLICE + lane;
-  const bool active = c < m.ncv && m.color[c] == color && st.case_active[m.case_of[c]];
-  const int N = m.ncv;
-  BT acc = 0;
-  if (active) {
-    acc = (BT)st.b[(size_t)B * c + row];
-    const BT* O = (const BT*)st.O;
-    for (int j = m.ell_off[slice]; j < m.ell_off[slice + 1]; j++) {
-      int nb = m.ell_nb[(size_t)j * SLICE + lane];
-      const BT* Ob = O + ((size_t)j * B * B + B * row) * SLICE + lane;
-      BT s = 0;
-      for (int k = 0; k < B; k++) s += Ob[k * SLICE] * x[(size_t)k * N + nb];
-      acc -= s;
-    }
-  }
-  sacc[row][lane] = acc;
-  __syncthreads();
-  if (active) {
-    const BT* Di = (const BT*)st.Dinv;
-    BT s = 0;
-    for (int k = 0; k < B; k++) s += Di[(size_t)(B * row + k) * N + c] * sacc[k][lane];
-    x[(size_t)row * N + c] = s;
-  }
-}
-
 // runBackwardEulerCoupled update (JoeWithModels.cpp:4497-4517): Q += dq, then
 // phi_s = clip((phi_s * (rho_new - dq0) + dq_{5+s}) / rho_new); dq kept in st.dq
 template <typename BT, int NS>
@@ -1297,23 +1233,8 @@ void launch_flux6(const Mesh& m, const Params& p, State& st, Turb& t, int implic
 }
 template <typename BT, int B>
 static void relax_c(const Mesh& m, State& st, int sgs, int sweeps, cudaStream_t s) {
-  if (sgs) {
-    cudaMemsetAsync(st.x0, 0, B * (size_t)m.ncv * sizeof(BT), s);
-    for (int it = 0; it < sweeps; it++)
-      for (int q = 0; q < m.ncolors; q++) {
-        int col = (it % 2 == 0) ? q : m.ncolors - 1 - q;
-        const bool lists = m.color_slices != nullptr;
-        const int* sl = lists ? m.color_slices + m.color_slice_off[col] : nullptr;
-        const int g = lists ? m.color_slice_off[col + 1] - m.color_slice_off[col] : m.nslices;
-        if (g > 0) k_gs_c<BT, B><<<g, B * SLICE, 0, s>>>(m, st, (BT*)st.x0, col, sl);
-      }
-  } else {
-    for (int it = 0; it < sweeps; it++) {
-      void* xin = (it % 2 == 0) ? st.x1 : st.x0;
-      void* xout = (it % 2 == 0) ? st.x0 : st.x1;
-      k_jacobi_c<BT, B><<<m.nslices, B * SLICE, 0, s>>>(m, st, (const BT*)xin, (BT*)xout, it == 0);
-    }
-  }
+  if (sgs) sweep_sgs<BT, B>(m, st, sweeps, s);
+  else sweep_jacobi<BT, B>(m, st, sweeps, s);
 }
 void launch_relax6(const Mesh& m, const Params& p, State& st, int sgs, int sweeps, int bs, cudaStream_t s) {
   if (bs == 7) {

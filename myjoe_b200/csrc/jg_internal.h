@@ -61,6 +61,7 @@ struct Mesh {
   int ell_rows;
   const uint8_t* color;    // [N] colour of the cell (no two neighbours share one)
   int ncolors;
+  int color_proper;        // 1: no internal face joins two cells of one colour (or a cell to itself)
   // per colour q (q < MAX_COLOR_LISTS): the slices holding a cell of that colour are
   // color_slices[color_slice_off[q] .. color_slice_off[q+1]) (host-side offsets; no lists when
   // ncolors > MAX_COLOR_LISTS: every colour pass covers every slice)
@@ -273,7 +274,8 @@ struct Lines {
   double* v;       // [off[nlines]][5]
   // LINE relaxation (B x B blocks in the matrix precision)
   const uint8_t* on_line;     // [N] 1 on the cells of the lines
-  const uint8_t* ell_inline;  // [ell_rows*32] 1 where the ELL entry couples a cell to its line neighbour
+  const int* noff;            // [N] couplings of the cell that are not to its line neighbours: its first ELL columns
+  const int* off_end;         // [nslices] one past the last ELL row holding such a coupling of a cell of the slice
   void* binv;      // [off[nlines]][B*B]
   void* blow;      // [off[nlines]][B*B]
   void* bup;       // [off[nlines]][B*B]

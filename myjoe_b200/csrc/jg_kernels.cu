@@ -11,6 +11,7 @@
 #include "jg_cell.cuh"
 #include "jg_flux.cuh"
 #include "jg_internal.h"
+#include "jg_sweep.cuh"
 
 namespace jg {
 
@@ -674,40 +675,6 @@ __global__ void k_jst(Mesh m, Params p, State st) {
   for (int i = 0; i < 5; i++) J[3 + i] = lap[i];
 }
 
-// Block point relaxation, one warp per block row: a 160-thread block handles
-// one 32-cell slice; warp i computes row i of (b - O x) for the 32 cells
-// (coalesced ELL reads), the 5 rows meet in shared memory for the Dinv product.
-template <typename BT>
-__global__ void __launch_bounds__(160) k_jacobi2(Mesh m, State st, const BT* __restrict__ xin,
-                                                 BT* __restrict__ xout, int first) {
-  __shared__ BT sacc[5][SLICE];
-  const int row = threadIdx.x / SLICE, lane = threadIdx.x % SLICE;
-  const int slice = blockIdx.x;
-  const int c = slice * SLICE + lane;
-  const bool active = c < m.ncv && st.case_active[m.case_of[c]];
-  const int N = m.ncv;
-  BT acc = active ? (BT)st.b[5 * c + row] : (BT)0;
-  if (!first && active) {
-    const BT* O = (const BT*)st.O;
-    int j0 = m.ell_off[slice], j1 = m.ell_off[slice + 1];
-    for (int j = j0; j < j1; j++) {
-      int nb = m.ell_nb[(size_t)j * SLICE + lane];
-      const BT* Ob = O + ((size_t)j * 25 + 5 * row) * SLICE + lane;
-      BT s = 0;
-      for (int k = 0; k < 5; k++) s += Ob[k * SLICE] * xin[(size_t)k * N + nb];
-      acc -= s;
-    }
-  }
-  sacc[row][lane] = acc;
-  __syncthreads();
-  if (active) {
-    const BT* Di = (const BT*)st.Dinv;
-    BT s = 0;
-    for (int k = 0; k < 5; k++) s += Di[(size_t)(5 * row + k) * N + c] * sacc[k][lane];
-    xout[(size_t)row * N + c] = s;
-  }
-}
-
 // residual history entry: sum of the per-block partials in block order
 __global__ void k_resid_final(State st, int nblk, int hist_from_ctrl) {
   __shared__ double s[5][256];
@@ -821,42 +788,6 @@ __global__ void __launch_bounds__(128) k_jacobi(Mesh m, State st, const BT* __re
     BT s = 0;
     for (int k = 0; k < 5; k++) s += Di[(size_t)(5 * i + k) * N + c] * acc[k];
     xout[(size_t)i * N + c] = s;
-  }
-}
-
-// Multicolour block Gauss-Seidel pass over one colour, in place: the cells of
-// a colour have no neighbours of the same colour, so each reads the latest
-// values of the others.  Same row-parallel layout as k_jacobi2.
-// slices (may be null: every slice): the slices that hold a cell of this colour
-template <typename BT>
-__global__ void __launch_bounds__(160) k_gs2(Mesh m, State st, BT* __restrict__ x, int color,
-                                             const int* __restrict__ slices) {
-  __shared__ BT sacc[5][SLICE];
-  const int row = threadIdx.x / SLICE, lane = threadIdx.x % SLICE;
-  const int slice = slices ? slices[blockIdx.x] : blockIdx.x;
-  const int c = slice * SLICE + lane;
-  const bool active = c < m.ncv && m.color[c] == color && st.case_active[m.case_of[c]];
-  const int N = m.ncv;
-  BT acc = 0;
-  if (active) {
-    acc = (BT)st.b[5 * c + row];
-    const BT* O = (const BT*)st.O;
-    int j0 = m.ell_off[slice], j1 = m.ell_off[slice + 1];
-    for (int j = j0; j < j1; j++) {
-      int nb = m.ell_nb[(size_t)j * SLICE + lane];
-      const BT* Ob = O + ((size_t)j * 25 + 5 * row) * SLICE + lane;
-      BT s = 0;
-      for (int k = 0; k < 5; k++) s += Ob[k * SLICE] * x[(size_t)k * N + nb];
-      acc -= s;
-    }
-  }
-  sacc[row][lane] = acc;
-  __syncthreads();
-  if (active) {
-    const BT* Di = (const BT*)st.Dinv;
-    BT s = 0;
-    for (int k = 0; k < 5; k++) s += Di[(size_t)(5 * row + k) * N + c] * sacc[k][lane];
-    x[(size_t)row * N + c] = s;
   }
 }
 
@@ -1219,34 +1150,23 @@ void launch_grad_coupled(const Mesh& m, const Params& p, State& st, cudaStream_t
 }
 // both sweep kernels do the same arithmetic in the same order (bit-identical results)
 void launch_jacobi(const Mesh& m, const Params& p, State& st, int sweeps, cudaStream_t s) {
+  if (p.relax_variant != 1) {
+    if (p.fp32) sweep_jacobi<float, 5>(m, st, sweeps, s);
+    else sweep_jacobi<double, 5>(m, st, sweeps, s);
+    return;
+  }
   for (int it = 0; it < sweeps; it++) {
     void* xin = (it % 2 == 0) ? st.x1 : st.x0;
     void* xout = (it % 2 == 0) ? st.x0 : st.x1;
-    if (p.relax_variant == 1) {
-      if (p.fp32)
-        k_jacobi<float><<<grid_for(m.ncv, TB), TB, 0, s>>>(m, st, (const float*)xin, (float*)xout, it == 0);
-      else
-        k_jacobi<double><<<grid_for(m.ncv, TB), TB, 0, s>>>(m, st, (const double*)xin, (double*)xout, it == 0);
-    } else if (p.fp32) {
-      k_jacobi2<float><<<m.nslices, 5 * SLICE, 0, s>>>(m, st, (const float*)xin, (float*)xout, it == 0);
-    } else {
-      k_jacobi2<double><<<m.nslices, 5 * SLICE, 0, s>>>(m, st, (const double*)xin, (double*)xout, it == 0);
-    }
+    if (p.fp32)
+      k_jacobi<float><<<grid_for(m.ncv, TB), TB, 0, s>>>(m, st, (const float*)xin, (float*)xout, it == 0);
+    else
+      k_jacobi<double><<<grid_for(m.ncv, TB), TB, 0, s>>>(m, st, (const double*)xin, (double*)xout, it == 0);
   }
 }
 void launch_sgs(const Mesh& m, const Params& p, State& st, int sweeps, cudaStream_t s) {
-  size_t bytes = 5 * (size_t)m.ncv * (p.fp32 ? sizeof(float) : sizeof(double));
-  cudaMemsetAsync(st.x0, 0, bytes, s);
-  for (int it = 0; it < sweeps; it++)
-    for (int q = 0; q < m.ncolors; q++) {
-      int col = (it % 2 == 0) ? q : m.ncolors - 1 - q;  // forward, then backward colour order
-      const bool lists = m.color_slices != nullptr;
-      const int* sl = lists ? m.color_slices + m.color_slice_off[col] : nullptr;
-      const int g = lists ? m.color_slice_off[col + 1] - m.color_slice_off[col] : m.nslices;
-      if (g == 0) continue;
-      if (p.fp32) k_gs2<float><<<g, 5 * SLICE, 0, s>>>(m, st, (float*)st.x0, col, sl);
-      else k_gs2<double><<<g, 5 * SLICE, 0, s>>>(m, st, (double*)st.x0, col, sl);
-    }
+  if (p.fp32) sweep_sgs<float, 5>(m, st, sweeps, s);
+  else sweep_sgs<double, 5>(m, st, sweeps, s);
 }
 void launch_dq_from_x(const Mesh& m, const Params& p, State& st, const void* x, cudaStream_t s) {
   if (p.fp32)

@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "jg_internal.h"
+#include "jg_sweep.cuh"
 
 namespace jg {
 
@@ -277,7 +278,7 @@ void launch_line_precond(const Mesh& m, const State& st, const Lines& L, const d
 // LINE relaxation: block line-Jacobi sweeps for B x B blocks (B = 5, 6, 7) in
 // the matrix precision BT.  A sweep is x' = T^-1 (b - (A - T) x), T the
 // block-tridiagonal part of A along the lines (the block diagonal elsewhere):
-//   k_lrelax_rhs: per cell r = b - sum of the off-diagonal blocks that are not
+//   k_sweep (LINE): per cell r = b - sum of the off-diagonal blocks that are not
 //                 a line coupling times x; off the lines x' = Dinv r, on the
 //                 lines r is left in x' for
 //   k_lsolve:     the block Thomas substitutions of each line, in place.
@@ -406,44 +407,6 @@ __global__ void __launch_bounds__(32 * LW) k_lfactor(Mesh m, State st, Lines L) 
     for (int t = 0; t < EP; t++)
       if (lane + 32 * t < BB) b[lane + 32 * t] = bn[t];
     __syncwarp();
-  }
-}
-
-// one block per 32-cell slice, B rows x 32 lanes (the k_jacobi_c layout)
-template <typename BT, int B>
-__global__ void __launch_bounds__(B * 32) k_lrelax_rhs(Mesh m, State st, Lines L, const BT* __restrict__ xin,
-                                                       BT* __restrict__ xout, int first) {
-  __shared__ BT sacc[B][SLICE];
-  const int row = threadIdx.x / SLICE, lane = threadIdx.x % SLICE;
-  const int slice = blockIdx.x;
-  const int c = slice * SLICE + lane;
-  const bool active = c < m.ncv;
-  const int N = m.ncv;
-  BT acc = active ? (BT)st.b[(size_t)B * c + row] : (BT)0;
-  if (!first && active) {
-    const BT* O = (const BT*)st.O;
-    for (int j = m.ell_off[slice]; j < m.ell_off[slice + 1]; j++) {
-      if (L.ell_inline[(size_t)j * SLICE + lane]) continue;
-      int nb = m.ell_nb[(size_t)j * SLICE + lane];
-      const BT* Ob = O + ((size_t)j * B * B + B * row) * SLICE + lane;
-      BT s = 0;
-#pragma unroll
-      for (int k = 0; k < B; k++) s += Ob[k * SLICE] * xin[(size_t)k * N + nb];
-      acc -= s;
-    }
-  }
-  sacc[row][lane] = acc;
-  __syncthreads();
-  if (active) {
-    if (L.on_line[c]) {
-      xout[(size_t)row * N + c] = acc;
-    } else {
-      const BT* Di = (const BT*)st.Dinv;
-      BT s = 0;
-#pragma unroll
-      for (int k = 0; k < B; k++) s += Di[(size_t)(B * row + k) * N + c] * sacc[k][lane];
-      xout[(size_t)row * N + c] = s;
-    }
   }
 }
 
@@ -600,7 +563,11 @@ void line_relax(const Mesh& m, State& st, const Lines& L, int sweeps, cudaStream
   for (int it = 0; it < sweeps; it++) {
     BT* xin = (BT*)((it % 2 == 0) ? st.x1 : st.x0);
     BT* xout = (BT*)((it % 2 == 0) ? st.x0 : st.x1);
-    k_lrelax_rhs<BT, B><<<m.nslices, B * SLICE, 0, s>>>(m, st, L, xin, xout, it == 0);
+    // two columns at a time: most line cells have three or four couplings off their line.  The passes
+    // and substitutions are plain launches: as programmatic dependents they measured 4-5% slower
+    // (a pass's early blocks take the SMs of the substitutions, which are a chain of latencies)
+    k_sweep<BT, B, SWEEP_LINE, 2, sizeof(BT) == 4 ? 1600 / (B * SLICE) : 1>
+        <<<m.nslices, B * SLICE, 0, s>>>(m, st, xin, xout, it == 0, -1, nullptr, L.on_line, L.noff, L.off_end);
     if (L.nlines) k_lsolve<BT, B><<<(L.nlines + LW * LPW - 1) / (LW * LPW), 32 * LW, 0, s>>>(m, L, xout);
   }
 }
