@@ -333,7 +333,8 @@ int jg_batch_set_active(jg_case_t *h, int case_id, int active);
  * lanes per cell with registers for two 128-thread blocks per SM, or
  * JG_FLUX_CL1_3BLK: one lane, registers capped for three blocks per SM -- or
  * split (flux_cl = JG_FLUX_SPLIT + FL, FL = 1, 2, 4 or 8; the default is
- * JG_FLUX_SPLIT + 4): a residual kernel with FL lanes per cell and a Jacobian
+ * JG_FLUX_SPLIT + 4): the residual (a thread per face forms its flux, a thread
+ * per cell sums them; the same kernels for every FL) and a Jacobian
  * kernel (one thread per cell, the face matrices formed row by row) on two
  * streams.  Second: the kernel of the 5x5 Jacobi sweep (0: a block per 32-cell
  * slice, a thread per block row, the default; 1: a thread per cell).

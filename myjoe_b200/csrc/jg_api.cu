@@ -189,6 +189,19 @@ static int download_rows(jg_case* h, const double* dev, double* host, const std:
   return JG_OK;
 }
 
+// the same for w doubles at the front of each device record of `stride` doubles
+static int download_fields(jg_case* h, const double* dev, size_t stride, double* host, const std::vector<int>& perm,
+                           size_t n, size_t w) {
+  std::vector<double> tmp(perm.empty() ? 0 : n * w);
+  double* to = perm.empty() ? host : tmp.data();
+  if (n)
+    CK(cudaMemcpy2DAsync(to, w * sizeof(double), dev, stride * sizeof(double), w * sizeof(double), n,
+                         cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaStreamSynchronize(h->stream));
+  if (!perm.empty()) rows_to_caller(perm, tmp.data(), host, n, w, 1);
+  return JG_OK;
+}
+
 // the caller's host rows -> a device array of the handle (synchronous: the caller's array may go away)
 static int upload_rows(jg_case* h, double* dev, const double* host, const std::vector<int>& perm, size_t n,
                        size_t w, size_t nblk = 1) {
@@ -240,6 +253,7 @@ static Params make_params(const jg_params& q) {
   p.gamma = q.gamma;
   p.R = q.R_gas;
   p.cp = p.gamma * p.R / (p.gamma - 1.0);
+  p.igm1 = 1.0 / (p.gamma - 1.0);
   for (int i = 0; i < 3; i++) p.gravity[i] = q.gravity[i];
   p.has_gravity = q.gravity[0] != 0.0 || q.gravity[1] != 0.0 || q.gravity[2] != 0.0;
   p.Pr = q.Pr;
@@ -572,9 +586,11 @@ static int build(jg_case* h, const jg_mesh* mesh, const jg_params* q) {
   RC(upload(h, &m.fa_n, mesh->fa_normal, 3 * (size_t)nfa));
   RC(upload(h, &m.cvofa, mesh->cvofa, 2 * (size_t)nfa));
   {
-    double *fu = nullptr, *fs = nullptr;
-    RC(dmalloc(h, &fu, 4 * (size_t)nfa));
+    double *xv = nullptr, *fu = nullptr, *fs = nullptr;
+    RC(dmalloc(h, &xv, 4 * (size_t)N));
+    RC(dmalloc(h, &fu, 8 * (size_t)nfa));
     RC(dmalloc(h, &fs, 4 * (size_t)(nfa - nfa_b)));
+    m.xv = xv;
     m.fa_u = fu;
     m.fa_s = fs;
   }
@@ -594,7 +610,7 @@ static int build(jg_case* h, const jg_mesh* mesh, const jg_params* q) {
   RC(upload(h, &m.color, color.data(), color.size()));
   m.ncolors = ncolors;
   m.color_proper = proper;
-  launch_face_geo(m, (double*)m.fa_u, (double*)m.fa_s, h->stream);
+  launch_geo(m, (double*)m.xv, (double*)m.fa_u, (double*)m.fa_s, h->stream);
   CKL();
   // device state
   State& st = h->st;
@@ -604,15 +620,16 @@ static int build(jg_case* h, const jg_mesh* mesh, const jg_params* q) {
   RC(dmalloc(h, &st.bfa, 8 * (size_t)nfa_b));
   RC(dmalloc(h, &st.mul_fa, (size_t)nfa));
   RC(dmalloc(h, &st.lam_fa, (size_t)nfa));
-  RC(dmalloc(h, &st.gu, 9 * (size_t)N));
+  RC(dmalloc(h, &st.gu, GS * (size_t)N));
   int separate = h->p.viscous && h->p.second_order && !h->p.visc_limiter && h->p.limiter && bs == 5;
-  if (separate) RC(dmalloc(h, &st.guv, 9 * (size_t)N));
+  if (separate) RC(dmalloc(h, &st.guv, GS * (size_t)N));
   else st.guv = st.gu;
-  RC(dmalloc(h, &st.grho, 3 * (size_t)N));
-  RC(dmalloc(h, &st.gp, 3 * (size_t)N));
-  RC(dmalloc(h, &st.gh, 3 * (size_t)N));
+  st.grho = st.gu + 9;
+  st.gp = st.gu + 12;
+  RC(dmalloc(h, &st.gh, GHS * (size_t)N));
   RC(dmalloc(h, &st.local_dt, (size_t)N));
   RC(dmalloc(h, &st.rhs, bs * (size_t)N));
+  if (bs == 5) RC(dmalloc(h, &st.ff, (h->p.viscous ? 12 : 8) * (size_t)nfa));
   st.shock_flag = nullptr;
   if (q->flux == JG_FLUX_AUSMDV && q->shock_fix != JG_SHOCK_FIX_NONE)
     RC(dmalloc(h, &st.shock_flag, (size_t)N));
@@ -844,14 +861,14 @@ static size_t footprint(const jg_mesh* mesh, const jg_params* q, const std::vect
   const size_t nz = std::max(1, mesh->nzones);
   const size_t a[] = {
       // mesh
-      3 * N * d, N * d, 3 * nfa * d, 3 * nfa * d, 2 * nfa * i, 4 * nfa * d, std::max<size_t>(4 * (nfa - nfa_b), 1) * d,
+      3 * N * d, N * d, 3 * nfa * d, 3 * nfa * d, 2 * nfa * i, 4 * N * d, 8 * nfa * d, std::max<size_t>(4 * (nfa - nfa_b), 1) * d,
       (N + 1) * i, (size_t)fi[N] * sizeof(Slot),
       (N + 1) * i, nbs * i, 3 * nbs * d, (N + 1) * i, std::max<size_t>(nbslot, 1) * i, 3 * nfa_b * d,
       nfa_b * i, nz * sizeof(DevZone), (nslices + 1) * i, rows * SLICE * i, rows * SLICE, N,
       // state
-      5 * N * d, 8 * N * d, 8 * nfa_b * d, nfa * d, nfa * d, 9 * N * d,
-      (q->mu_ref > 0.0 && q->second_order && !q->visc_limiter && q->limiter && bs == 5) ? 9 * N * d : 0,
-      3 * N * d, 3 * N * d, 3 * N * d, N * d, bs * N * d, bs * N * d,
+      5 * N * d, 8 * N * d, 8 * nfa_b * d, nfa * d, nfa * d, GS * N * d,
+      (q->mu_ref > 0.0 && q->second_order && !q->visc_limiter && q->limiter && bs == 5) ? GS * N * d : 0,
+      GHS * N * d, bs == 5 ? (q->mu_ref > 0.0 ? 12 : 8) * nfa * d : 0, N * d, bs * N * d, bs * N * d,
       b2 * N * e, b2 * N * e, rows * b2 * SLICE * e, bs * N * e, bs * N * e, bs * N * d,
       (5 * (size_t)grid_for((int)N, 16) + 5 * (size_t)grid_for((int)N, 256) + 16) * d, 16 * d, 4 * i,
       bs * 64 * d, 2 * i, N * i, 1 * i, 1,
@@ -1398,10 +1415,10 @@ int jg_get_gradients(jg_case_t* h, double* grad_u, double* grad_rho, double* gra
   // the reference's grad_u after calcRhs: the viscous pass overwrites it (unlimited when VISC_LIMITER=NO)
   const double* gu = h->p.viscous ? h->st.guv : h->st.gu;
   const std::vector<int>& perm = h->rn.cell_old;
-  if (grad_u) RC(download_rows(h, gu, grad_u, perm, N, 9));
-  if (grad_rho) RC(download_rows(h, h->st.grho, grad_rho, perm, N, 3));
-  if (grad_p) RC(download_rows(h, h->st.gp, grad_p, perm, N, 3));
-  if (grad_h) RC(download_rows(h, h->st.gh, grad_h, perm, N, 3));
+  if (grad_u) RC(download_fields(h, gu, GS, grad_u, perm, N, 9));
+  if (grad_rho) RC(download_fields(h, h->st.grho, GS, grad_rho, perm, N, 3));
+  if (grad_p) RC(download_fields(h, h->st.gp, GS, grad_p, perm, N, 3));
+  if (grad_h) RC(download_fields(h, h->st.gh, GHS, grad_h, perm, N, 3));
   return JG_OK;
 }
 

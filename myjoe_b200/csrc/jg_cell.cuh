@@ -17,24 +17,20 @@ __device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefe
 // the face loop's reads of a neighbour cell c, prefetched a face ahead: its state, primitives,
 // centre, gradients (and the viscous gradients)
 __device__ __forceinline__ void prefetch_cell(const State& st, const Mesh& m, int c, bool visc) {
-  prefetch_l1(&st.q[5 * c]);
-  prefetch_l1(&st.prim[8 * c]);
-  prefetch_l1(&m.x_cv[3 * c]);
-  prefetch_l1(&st.grho[3 * c]);
-  prefetch_l1(&st.gp[3 * c]);
-  prefetch_l1(&st.gu[9 * c]);
+  prefetch_l1(&st.prim[(size_t)8 * c]);
+  prefetch_l1(&m.xv[(size_t)4 * c]);
+  prefetch_l1(&st.gu[(size_t)GS * c]);
   if (visc) {
-    prefetch_l1(&st.guv[9 * c]);
-    prefetch_l1(&st.gh[3 * c]);
+    prefetch_l1(&st.guv[(size_t)GS * c]);
+    prefetch_l1(&st.gh[(size_t)GHS * c]);
   }
 }
 
 // the Jacobian kernel's reads of a neighbour cell c: its state and primitives (and the viscous
 // gradient the viscous matrices' stress needs)
 __device__ __forceinline__ void prefetch_cell_jac(const State& st, int c, bool visc) {
-  prefetch_l1(&st.q[5 * c]);
-  prefetch_l1(&st.prim[8 * c]);
-  if (visc) prefetch_l1(&st.guv[9 * c]);
+  prefetch_l1(&st.prim[(size_t)8 * c]);
+  if (visc) prefetch_l1(&st.guv[(size_t)GS * c]);
 }
 
 // sourceHook / sourceHookCoupled (JoeWithModels.h:111-152): gravity in cell c's momentum and
@@ -59,26 +55,39 @@ __device__ __forceinline__ void gravity_diag(const Params& p, const Mesh& m, int
 
 // the unit normal and area of face f (normVec3d of fa_normal, formed once per mesh by k_face_geo)
 __device__ __forceinline__ void unit_normal(const Mesh& m, int f, double nV[3], double& area) {
-  const double* u = &m.fa_u[4 * f];
+  double u[4];
+  ld4(u, &m.fa_u[(size_t)8 * f]);
   for (int i = 0; i < 3; i++) nV[i] = u[i];
   area = u[3];
+}
+// the vector from cell c's centre to face f's
+__device__ __forceinline__ void cell_to_face(const Mesh& m, int c, int f, double r[3]) {
+  double x[4], xc[4];
+  ld4(x, &m.fa_u[(size_t)8 * f + 4]);
+  ld4(xc, &m.xv[(size_t)4 * c]);
+  for (int i = 0; i < 3; i++) r[i] = x[i] - xc[i];
 }
 
 // the unit vector from an internal face's cvofa[f][0] centre to its cvofa[f][1] centre and its
 // length (the viscous flux's sVec and smag, JoeWithModels.cpp:3626-3629)
 __device__ __forceinline__ void cell_to_cell(const Mesh& m, int f, double sV[3], double& smag) {
-  const double* s = &m.fa_s[4 * (f - m.nfa_b)];
+  double s[4];
+  ld4(s, &m.fa_s[(size_t)4 * (f - m.nfa_b)]);
   for (int i = 0; i < 3; i++) sV[i] = s[i];
   smag = s[3];
 }
 
 __device__ __forceinline__ FState cell_fstate(const Params& p, const State& st, int c) {
   FState s;
-  s.rho = st.q[5 * c];
-  for (int i = 0; i < 3; i++) s.u[i] = st.prim[8 * c + i];
-  s.p = st.prim[8 * c + 3];
+  double a[4], b[4];
+  ld4(a, &st.prim[(size_t)8 * c]);
+  ld4(b, &st.prim[(size_t)8 * c + 4]);
+  for (int i = 0; i < 3; i++) s.u[i] = a[i];
+  s.p = a[3];
   s.gam = p.gamma;
-  s.h = st.prim[8 * c + 5];
+  s.ig = p.igm1;
+  s.h = b[1];
+  s.rho = b[3];
   return s;
 }
 
@@ -87,19 +96,15 @@ __device__ __forceinline__ FState cell_fstate(const Params& p, const State& st, 
 __device__ __forceinline__ FState recon(const Mesh& m, const Params& p, const State& st, int c, int f) {
   FState s = cell_fstate(p, st, c);
   if (!p.second_order) return s;
-  double r0[3], gr[3], gp[3], gu[9];
-  for (int i = 0; i < 3; i++) {
-    r0[i] = m.x_fa[3 * f + i] - m.x_cv[3 * c + i];
-    gr[i] = st.grho[3 * c + i];
-    gp[i] = st.gp[3 * c + i];
-  }
-  for (int i = 0; i < 9; i++) gu[i] = st.gu[9 * c + i];
-  double rr = s.rho + dot3(r0, gr);
-  double pp = s.p + dot3(r0, gp);
+  double r0[3], g[GS];
+  for (int i = 0; i < GS; i += 4) ld4(g + i, &st.gu[(size_t)GS * c + i]);
+  cell_to_face(m, c, f, r0);
+  double rr = s.rho + dot3(r0, g + 9);
+  double pp = s.p + dot3(r0, g + 12);
   if ((pp <= 0.0) || (rr <= 0.0)) return s;  // first order: the cell's own h is calcThermoProp_p of (p, rho)
   s.rho = rr;
   s.p = pp;
-  for (int i = 0; i < 3; i++) s.u[i] += dot3(r0, &gu[3 * i]);
+  for (int i = 0; i < 3; i++) s.u[i] += dot3(r0, &g[3 * i]);
   const double T = pp / (rr * p.R);  // calcThermoProp_p at the face
   s.h = p.cp * T;
   return s;
@@ -107,14 +112,17 @@ __device__ __forceinline__ FState recon(const Mesh& m, const Params& p, const St
 
 __device__ __forceinline__ VSide cell_vside(const Params& p, const State& st, int c) {
   VSide v;
-  v.rho = st.q[5 * c];
-  for (int i = 0; i < 3; i++) v.u[i] = st.prim[8 * c + i];
-  v.h = st.prim[8 * c + 5];
-  v.T = st.prim[8 * c + 4];
+  double a[4], b[4];
+  ld4(a, &st.prim[(size_t)8 * c]);
+  ld4(b, &st.prim[(size_t)8 * c + 4]);
+  for (int i = 0; i < 3; i++) v.u[i] = a[i];
+  v.T = b[0];
+  v.h = b[1];
+  v.rho = b[3];
   v.R = p.R;
   v.gam = p.gamma;
-  v.gu = &st.guv[9 * c];
-  v.gh = &st.gh[3 * c];
+  v.gu = &st.guv[(size_t)GS * c];
+  v.gh = &st.gh[(size_t)GHS * c];
   return v;
 }
 

@@ -176,7 +176,7 @@ __device__ __forceinline__ double face_avg_c(const Mesh& m, const double* phi, i
 __global__ void k_turb_cell(Mesh m, State st, Turb t) {
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.ncv) return;
-  const double* g = &st.gu[9 * c];
+  const double* g = &st.gu[GS * c];
   double div = g[0] + g[4] + g[8];
   double sm = 0.0, vm = 0.0;
   for (int i = 0; i < 3; i++)
@@ -531,6 +531,7 @@ __device__ __forceinline__ FState fstate_c(const CState<NS>& s) {
   for (int i = 0; i < 3; i++) f.u[i] = s.u[i];
   f.p = s.p;
   f.gam = s.gam;
+  f.ig = 1.0 / (s.gam - 1.0);
   f.h = s.h + s.k;
   return f;
 }
@@ -796,13 +797,13 @@ __device__ __forceinline__ CState<NS> recon_c(const Mesh& m, const Params& p, co
   if (!p.second_order) return s;
   double r0[3];
   for (int i = 0; i < 3; i++) r0[i] = m.x_fa[3 * f + i] - m.x_cv[3 * c + i];
-  double rr = s.rho + dot3(r0, &st.grho[3 * c]);
-  double pp = s.p + dot3(r0, &st.gp[3 * c]);
+  double rr = s.rho + dot3(r0, &st.grho[GS * c]);
+  double pp = s.p + dot3(r0, &st.gp[GS * c]);
   if ((pp <= 0.0) || (rr <= 0.0)) {
     pp = s.p;
     rr = s.rho;
   } else {
-    for (int i = 0; i < 3; i++) s.u[i] += dot3(r0, &st.gu[9 * c + 3 * i]);
+    for (int i = 0; i < 3; i++) s.u[i] += dot3(r0, &st.gu[GS * c + 3 * i]);
     for (int q = 0; q < NS; q++) s.sc[q] += dot3(r0, &t.grad_phi[((size_t)q * m.ncv + c) * 3]);
   }
   s.rho = rr;
@@ -826,8 +827,8 @@ __device__ __forceinline__ VSideC<NS> vcell_c(const Mesh& m, const State& st, co
     v.gs[q] = &t.grad_phi[((size_t)q * m.ncv + c) * 3];
   }
   v.k = sst ? v.sc[0] : 0.0;
-  v.gu = &st.gu[9 * c];
-  v.gh = &st.gh[3 * c];
+  v.gu = &st.gu[GS * c];
+  v.gh = &st.gh[GHS * c];
   return v;
 }
 // boundary-face state for the viscous flux; scalars and their gradients set by the caller
@@ -845,8 +846,8 @@ __device__ __forceinline__ VSideC<NS> vbfa_c(const State& st, const Params& p, i
     v.gs[q] = nullptr;
   }
   v.k = 0.0;
-  v.gu = &st.gu[9 * c];
-  v.gh = &st.gh[3 * c];
+  v.gu = &st.gu[GS * c];
+  v.gh = &st.gh[GHS * c];
   return v;
 }
 
@@ -1004,7 +1005,7 @@ __global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb
           }
         }
         if (z.kind == JG_BC_SYMMETRY) {
-          const double* g = &st.gu[9 * c];
+          const double* g = &st.gu[GS * c];
           double tmp = 2.0 / 3.0 * ((st.mul_fa[f] + st.mut_fa[f]) * (g[0] + g[4] + g[8]) + Bs.rho * Bs.k);
           for (int i = 0; i < 3; i++) rhs[1 + i] -= area * tmp * nV[i];
         } else {

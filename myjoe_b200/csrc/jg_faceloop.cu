@@ -1,10 +1,13 @@
 // jg_faceloop.cu -- the face loop (calcEulerFlux + calcViscousFluxNS,
-// JoeWithModels.cpp:2621-3855) as two kernels on two streams:
+// JoeWithModels.cpp:2621-3855) as a residual and a Jacobian part on two streams:
 //
-//  * k_res: the residual.  Second-order reconstruction at the face, the
-//    Riemann flux, the viscous flux; FL lanes per cell (lane l takes the cell's
-//    face slots l, l+FL, ...), the lanes' sums combined by a butterfly in a
-//    fixed order.  No Jacobian live set, so ~120 registers and many warps.
+//  * k_face_flux, k_res: the residual.  A thread per face forms the second-order
+//    reconstruction, the Riemann flux and the viscous flux once; a thread per cell
+//    then sums its faces' fluxes.  Bound by the latency of the gathers and of the
+//    FP64 chains, so the work is cut into the most threads with the fewest registers
+//    (80 inviscid, 104 viscous): a thread per cell and four slots evaluated every
+//    internal face twice.  300k cells HLLC 169 -> 84 + 38 us, the 49k-cell viscous Roe
+//    plate 46 -> 24 + 10 us.
 //  * k_jac: the Jacobian blocks, which the reference forms at the cell-centre
 //    states (JoeWithModels.cpp:3032-3102).  One thread per cell walks the
 //    cell's faces; each face's two matrices come one row at a time
@@ -13,9 +16,9 @@
 //    store per entry across the 32 cells of a slice).  The epilogue adds
 //    vol/dt, stores D and its inverse (ludeco / luinv).
 //
-// Both kernels are cell-centric: each face is evaluated from both of its
-// cells, in the face's own orientation, so the two cells obtain bit-identical
-// face fluxes and every row has a single writer (no atomics, deterministic).
+// Every row has a single writer (no atomics, deterministic); the Jacobian is
+// cell-centric: each face is evaluated from both of its cells, in the face's own
+// orientation.
 //
 // Lagged Jacobian (State::jac_lag > 1): k_jac runs only on the steps a case's
 // blocks are due; it keeps the face part of the diagonal in D0.  On the other
@@ -44,108 +47,114 @@ __device__ __forceinline__ bool jac_due(const State& st, int k) {
 // ---------------------------------------------------------------------------
 // residual
 // ---------------------------------------------------------------------------
-template <int FL>
-__device__ __forceinline__ double lanes_sum(double v) {
-#pragma unroll
-  for (int o = FL / 2; o >= 1; o /= 2) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-template <int KIND, int VISC, int FL>
-__global__ void __launch_bounds__(TB) k_res(Mesh m, Params p, State st, int for_step) {
-  const int t = threadIdx.x, lane = t % FL;
-  const int c = blockIdx.x * (TB / FL) + t / FL;
-  const bool active = c < m.ncv && st.case_active[m.case_of[c]];  // a frozen case keeps its arrays
-  double rhs[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  const int k0 = active ? m.slot_i[c] : 0, k1 = active ? m.slot_i[c + 1] : 0;
-  if (k0 + lane < k1) {
-    const int nb = m.slots[k0 + lane].nb;
-    if (nb >= 0) prefetch_cell(st, m, nb, VISC);
-  }
-  for (int k = k0 + lane; k < k1; k += FL) {
-    const Slot s = m.slots[k];
-    const int f = s.f;
-    if (k + FL < k1) {  // the next face's neighbour, a face ahead
-      const int nb = m.slots[k + FL].nb;
-      if (nb >= 0) prefetch_cell(st, m, nb, VISC);
+// The fluxes of one face, a thread per face, into ff[f]: internal faces the Euler flux (5) and, at
+// ff + 5, the viscous one (4), boundary faces their sum.  FF: doubles per face
+template <int VISC>
+constexpr int FF = VISC ? 12 : 8;
+template <int KIND, int VISC>
+__global__ void __launch_bounds__(TB, VISC ? 3 : 4) k_face_flux(Mesh m, Params p, State st) {
+  const int f = blockIdx.x * TB + threadIdx.x;
+  if (f >= m.nfa) return;
+  const int c0 = m.cvofa[2 * f], c1 = m.cvofa[2 * f + 1];
+  if (!st.case_active[m.case_of[c0]]) return;  // a frozen case keeps its arrays
+  double nV[3], area, F[FF<VISC>];
+  for (int i = 5; i < FF<VISC>; i++) F[i] = 0.0;
+  unit_normal(m, f, nV, area);
+  if (f >= m.nfa_b) {
+    {
+      const FState L = recon(m, p, st, c0, f), R = recon(m, p, st, c1, f);
+      euler_flux_t<KIND>(F, L, R, area, nV, face_opts<KIND>(p, st, c0, c1), KIND == 5 ? &st.jst[8 * c0] : nullptr,
+                         KIND == 5 ? &st.jst[8 * c1] : nullptr);
     }
-    double nV[3], area;
-    unit_normal(m, f, nV, area);
-    if (s.nb >= 0) {
-      const int c0 = s.side == 0 ? c : s.nb;
-      const int c1 = s.side == 0 ? s.nb : c;
-      const double sg = s.side == 0 ? -1.0 : 1.0;  // residual sign of this cell
-      {
-        FState L = recon(m, p, st, c0, f), R = recon(m, p, st, c1, f);
-        double F[5];
-        euler_flux_t<KIND>(F, L, R, area, nV, face_opts<KIND>(p, st, c0, c1), KIND == 5 ? &st.jst[8 * c0] : nullptr,
-                           KIND == 5 ? &st.jst[8 * c1] : nullptr);
-        for (int i = 0; i < 5; i++) rhs[i] += sg * F[i];
-      }
-      if (VISC) {
-        VSide v0 = cell_vside(p, st, c0), v1 = cell_vside(p, st, c1);
-        double sV[3], smag;
-        cell_to_cell(m, f, sV, smag);
-        double ufa[3] = {0.5 * (v0.u[0] + v1.u[0]), 0.5 * (v0.u[1] + v1.u[1]), 0.5 * (v0.u[2] + v1.u[2])};
-        double Fu[3], FE;
-        VFace vf;
-        visc_flux(Fu, FE, vf, v0, v1, st.mul_fa[f], 0.0, st.lam_fa[f], p.PrTurb, ufa, area, nV, smag, sV);
-        for (int i = 0; i < 3; i++) rhs[1 + i] += sg * Fu[i];
-        rhs[4] += sg * FE;
+    if (VISC) {
+      VSide v0 = cell_vside(p, st, c0), v1 = cell_vside(p, st, c1);
+      double sV[3], smag;
+      cell_to_cell(m, f, sV, smag);
+      double ufa[3] = {0.5 * (v0.u[0] + v1.u[0]), 0.5 * (v0.u[1] + v1.u[1]), 0.5 * (v0.u[2] + v1.u[2])};
+      double Fu[3], FE;
+      VFace vf;
+      visc_flux(Fu, FE, vf, v0, v1, st.mul_fa[f], 0.0, st.lam_fa[f], p.PrTurb, ufa, area, nV, smag, sV);
+      for (int i = 0; i < 3; i++) F[5 + i] = Fu[i];
+      F[8] = FE;
+    }
+  } else {
+    const DevZone& z = m.zones[m.bzone[f]];
+    double bb[8];
+    ld4(bb, &st.bfa[(size_t)8 * f]);
+    ld4(bb + 4, &st.bfa[(size_t)8 * f + 4]);
+    FState B;
+    B.rho = bb[0]; B.u[0] = bb[1]; B.u[1] = bb[2]; B.u[2] = bb[3]; B.p = bb[4]; B.gam = p.gamma; B.ig = p.igm1; B.h = bb[6];
+    const int fob = bnd_opts<KIND>(p);
+    const double* jb = KIND == 5 ? &st.jst[8 * c0] : nullptr;
+    double r[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // the face's share of the cell's residual
+    if (z.kind == JG_BC_SYMMETRY || z.kind == JG_BC_WALL) {
+      euler_flux_t<KIND>(F, B, B, area, nV, fob, jb, jb);
+      if (z.kind == JG_BC_SYMMETRY && p.symm_bc == JG_SYMM_ANALYTICAL) {
+        for (int i = 0; i < 3; i++) r[1 + i] -= bb[4] * nV[i] * area;
+      } else {
+        for (int i = 0; i < 5; i++) r[i] -= F[i];
       }
     } else {
-      // boundary face (the cell is cvofa[f][0])
-      const DevZone z = m.zones[m.bzone[f]];
-      const double* bb = &st.bfa[8 * f];
-      FState B;
-      B.rho = bb[0]; B.u[0] = bb[1]; B.u[1] = bb[2]; B.u[2] = bb[3]; B.p = bb[4]; B.gam = p.gamma; B.h = bb[6];
-      double F[5];
-      const int fob = bnd_opts<KIND>(p);
-      const double* jb = KIND == 5 ? &st.jst[8 * c] : nullptr;
-      if (z.kind == JG_BC_SYMMETRY || z.kind == JG_BC_WALL) {
-        euler_flux_t<KIND>(F, B, B, area, nV, fob, jb, jb);
-        if (z.kind == JG_BC_SYMMETRY && p.symm_bc == JG_SYMM_ANALYTICAL) {
-          for (int i = 0; i < 3; i++) rhs[1 + i] -= bb[4] * nV[i] * area;
-        } else {
-          for (int i = 0; i < 5; i++) rhs[i] -= F[i];
-        }
-      } else {
-        FState L = recon(m, p, st, c, f);
-        euler_flux_t<KIND>(F, L, B, area, nV, fob, jb, jb);
-        for (int i = 0; i < 5; i++) rhs[i] -= F[i];
-      }
-      if (VISC && z.kind != JG_BC_SYMMETRY) {
-        VSide v0 = cell_vside(p, st, c);
-        VSide v1;
-        v1.rho = bb[0]; v1.u[0] = bb[1]; v1.u[1] = bb[2]; v1.u[2] = bb[3];
-        v1.h = bb[6]; v1.T = bb[5]; v1.R = p.R; v1.gam = p.gamma;
-        v1.gu = v0.gu; v1.gh = v0.gh;
-        double sV[3], smag;
-        for (int i = 0; i < 3; i++) sV[i] = m.x_fa[3 * f + i] - m.x_cv[3 * c + i];
-        if (z.kind == JG_BC_WALL) {
-          smag = fabs(dot3(sV, nV));  // projected on the wall normal; nVec is used as sVec
-          for (int i = 0; i < 3; i++) sV[i] = nV[i];
-        } else {
-          smag = sqrt(dot3(sV, sV));
-          for (int i = 0; i < 3; i++) sV[i] /= smag;
-        }
-        double Fu[3], FE;
-        VFace vf;
-        visc_flux(Fu, FE, vf, v0, v1, st.mul_fa[f], 0.0, st.lam_fa[f], p.PrTurb, v1.u, area, nV, smag, sV);
-        for (int i = 0; i < 3; i++) rhs[1 + i] -= Fu[i];
-        rhs[4] -= FE;
-      }
+      const FState L = recon(m, p, st, c0, f);
+      euler_flux_t<KIND>(F, L, B, area, nV, fob, jb, jb);
+      for (int i = 0; i < 5; i++) r[i] -= F[i];
     }
+    if (VISC && z.kind != JG_BC_SYMMETRY) {
+      VSide v0 = cell_vside(p, st, c0);
+      VSide v1;
+      v1.rho = bb[0]; v1.u[0] = bb[1]; v1.u[1] = bb[2]; v1.u[2] = bb[3];
+      v1.h = bb[6]; v1.T = bb[5]; v1.R = p.R; v1.gam = p.gamma;
+      v1.gu = v0.gu; v1.gh = v0.gh;
+      double sV[3], smag;
+      cell_to_face(m, c0, f, sV);
+      if (z.kind == JG_BC_WALL) {
+        smag = fabs(dot3(sV, nV));  // projected on the wall normal; nVec is used as sVec
+        for (int i = 0; i < 3; i++) sV[i] = nV[i];
+      } else {
+        smag = sqrt(dot3(sV, sV));
+        for (int i = 0; i < 3; i++) sV[i] /= smag;
+      }
+      double Fu[3], FE;
+      VFace vf;
+      visc_flux(Fu, FE, vf, v0, v1, st.mul_fa[f], 0.0, st.lam_fa[f], p.PrTurb, v1.u, area, nV, smag, sV);
+      for (int i = 0; i < 3; i++) r[1 + i] -= Fu[i];
+      r[4] -= FE;
+    }
+    for (int i = 0; i < 5; i++) F[i] = -r[i];
   }
-  // the lanes of a cell share its activity, so every lane of the warp reaches the shuffles
-  if (FL > 1)
-    for (int i = 0; i < 5; i++) rhs[i] = lanes_sum<FL>(rhs[i]);
-  if (active && lane == 0) {
-    gravity_rhs(p, m, st, c, rhs);
-    for (int i = 0; i < 5; i++) st.rhs[5 * c + i] = rhs[i];
-    if (for_step)
-      for (int i = 0; i < 5; i++) st.b[5 * c + i] = p.under_relax * rhs[i];
+  double* o = &st.ff[(size_t)FF<VISC> * f];
+  for (int i = 0; i < FF<VISC>; i += 4) st4(o + i, F + i);
+}
+
+// The residual of a cell: its faces' fluxes summed over the face slots, every fourth slot into one of
+// four sums (the order of a four-lane loop over the slots), the sums as (0 + 2) + (1 + 3)
+template <int VISC>
+__global__ void __launch_bounds__(TB) k_res(Mesh m, Params p, State st, int for_step) {
+  const int c = blockIdx.x * TB + threadIdx.x;
+  if (c >= m.ncv || !st.case_active[m.case_of[c]]) return;
+  double v[4][5];
+  for (int t = 0; t < 4; t++)
+    for (int i = 0; i < 5; i++) v[t][i] = 0.0;
+  const int k0 = m.slot_i[c], k1 = m.slot_i[c + 1];
+  for (int k = k0; k < k1; k += 4) {
+#pragma unroll
+    for (int t = 0; t < 4; t++)
+      if (k + t < k1) {
+        const int4 s = *reinterpret_cast<const int4*>(&m.slots[k + t]);  // face, neighbour, side, column
+        const double* f = &st.ff[(size_t)FF<VISC> * s.x];
+        double F[FF<VISC>];
+        for (int i = 0; i < FF<VISC>; i += 4) ld4(F + i, f + i);
+        for (int i = 0; i < 5; i++) v[t][i] += s.z == 0 ? -F[i] : F[i];
+        if (VISC)
+          for (int i = 0; i < 4; i++) v[t][1 + i] += s.z == 0 ? -F[5 + i] : F[5 + i];
+      }
   }
+  double rhs[5];
+  for (int i = 0; i < 5; i++) rhs[i] = (v[0][i] + v[2][i]) + (v[1][i] + v[3][i]);
+  gravity_rhs(p, m, st, c, rhs);
+  for (int i = 0; i < 5; i++) st.rhs[(size_t)5 * c + i] = rhs[i];
+  if (for_step)
+    for (int i = 0; i < 5; i++) st.b[(size_t)5 * c + i] = p.under_relax * rhs[i];
 }
 
 // ---------------------------------------------------------------------------
@@ -230,7 +239,7 @@ __global__ void __launch_bounds__(TB, jac_min_blocks<BT, KIND>()) k_jac(Mesh m, 
       const DevZone z = m.zones[m.bzone[f]];
       const double* bb = &st.bfa[8 * f];
       FState B;
-      B.rho = bb[0]; B.u[0] = bb[1]; B.u[1] = bb[2]; B.u[2] = bb[3]; B.p = bb[4]; B.gam = p.gamma; B.h = bb[6];
+      B.rho = bb[0]; B.u[0] = bb[1]; B.u[1] = bb[2]; B.u[2] = bb[3]; B.p = bb[4]; B.gam = p.gamma; B.ig = p.igm1; B.h = bb[6];
       const FStateT<JT> Bt = fstate_as<JT>(B);
       const int fob = bnd_opts<KIND>(p);
       if (z.kind == JG_BC_SYMMETRY && p.symm_bc == JG_SYMM_ANALYTICAL) {
@@ -261,7 +270,7 @@ __global__ void __launch_bounds__(TB, jac_min_blocks<BT, KIND>()) k_jac(Mesh m, 
         v1.h = bb[6]; v1.T = bb[5]; v1.R = p.R; v1.gam = p.gamma;
         v1.gu = v0.gu; v1.gh = v0.gh;
         double sV[3], smag;
-        for (int i = 0; i < 3; i++) sV[i] = m.x_fa[3 * f + i] - m.x_cv[3 * c + i];
+        cell_to_face(m, c, f, sV);
         if (z.kind == JG_BC_WALL) {
           smag = fabs(dot3(sV, nV));
           for (int i = 0; i < 3; i++) sV[i] = nV[i];
@@ -322,29 +331,24 @@ __global__ void __launch_bounds__(TB) k_diag(Mesh m, State st) {
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-template <int KIND, int VISC>
-static void launch_res_kv(const Mesh& m, const Params& p, State& st, int fl, int for_step, cudaStream_t s) {
-  switch (fl) {
-    case 1: k_res<KIND, VISC, 1><<<grid_for(m.ncv, TB), TB, 0, s>>>(m, p, st, for_step); break;
-    case 2: k_res<KIND, VISC, 2><<<grid_for(m.ncv, TB / 2), TB, 0, s>>>(m, p, st, for_step); break;
-    case 4: k_res<KIND, VISC, 4><<<grid_for(m.ncv, TB / 4), TB, 0, s>>>(m, p, st, for_step); break;
-    default: k_res<KIND, VISC, 8><<<grid_for(m.ncv, TB / 8), TB, 0, s>>>(m, p, st, for_step); break;
-  }
-}
 template <int KIND>
-static void launch_res_k(const Mesh& m, const Params& p, State& st, int fl, int for_step, cudaStream_t s) {
-  if (p.viscous) launch_res_kv<KIND, 1>(m, p, st, fl, for_step, s);
-  else launch_res_kv<KIND, 0>(m, p, st, fl, for_step, s);
+static void launch_face_flux(const Mesh& m, const Params& p, State& st, cudaStream_t s) {
+  const int g = grid_for(m.nfa, TB);
+  if (g == 0) return;
+  if (p.viscous) k_face_flux<KIND, 1><<<g, TB, 0, s>>>(m, p, st);
+  else k_face_flux<KIND, 0><<<g, TB, 0, s>>>(m, p, st);
 }
-static void launch_res(const Mesh& m, const Params& p, State& st, int fl, int for_step, cudaStream_t s) {
+static void launch_res(const Mesh& m, const Params& p, State& st, int for_step, cudaStream_t s) {
   switch (p.flux) {
-    case JG_FLUX_ROE: launch_res_k<1>(m, p, st, fl, for_step, s); break;
-    case JG_FLUX_AUSM: launch_res_k<2>(m, p, st, fl, for_step, s); break;
-    case JG_FLUX_HAENEL: launch_res_k<3>(m, p, st, fl, for_step, s); break;
-    case JG_FLUX_AUSMDV: launch_res_k<4>(m, p, st, fl, for_step, s); break;
-    case JG_FLUX_JST: launch_res_k<5>(m, p, st, fl, for_step, s); break;
-    default: launch_res_k<0>(m, p, st, fl, for_step, s); break;
+    case JG_FLUX_ROE: launch_face_flux<1>(m, p, st, s); break;
+    case JG_FLUX_AUSM: launch_face_flux<2>(m, p, st, s); break;
+    case JG_FLUX_HAENEL: launch_face_flux<3>(m, p, st, s); break;
+    case JG_FLUX_AUSMDV: launch_face_flux<4>(m, p, st, s); break;
+    case JG_FLUX_JST: launch_face_flux<5>(m, p, st, s); break;
+    default: launch_face_flux<0>(m, p, st, s); break;
   }
+  if (p.viscous) k_res<1><<<grid_for(m.ncv, TB), TB, 0, s>>>(m, p, st, for_step);
+  else k_res<0><<<grid_for(m.ncv, TB), TB, 0, s>>>(m, p, st, for_step);
 }
 
 template <typename BT, int KIND>
@@ -380,25 +384,24 @@ static void launch_jacobian(const Mesh& m, const Params& p, State& st, int for_s
 void launch_flux(const Mesh& m, const Params& p, State& st, int implicit, int for_step, cudaStream_t s) {
   launch_face_sensors(m, p, st, s);
   if (!implicit) {
-    launch_res(m, p, st, flux_split(p, st) ? flux_split_lanes(p) : 8, for_step, s);
+    launch_res(m, p, st, for_step, s);
     return;
   }
   if (!flux_split(p, st)) {
     launch_flux_fused(m, p, st, for_step, s);
     return;
   }
-  const int fl = flux_split_lanes(p);
   if (st.aux && st.ev_fork && st.ev_join) {
     // the two kernels are independent: the Jacobian on the second stream, joined before the caller's next work
     cudaEventRecord(st.ev_fork, s);
     cudaStreamWaitEvent(st.aux, st.ev_fork, 0);
     launch_jacobian(m, p, st, for_step, st.aux);
-    launch_res(m, p, st, fl, for_step, s);
+    launch_res(m, p, st, for_step, s);
     cudaEventRecord(st.ev_join, st.aux);
     cudaStreamWaitEvent(s, st.ev_join, 0);
   } else {
     launch_jacobian(m, p, st, for_step, s);
-    launch_res(m, p, st, fl, for_step, s);
+    launch_res(m, p, st, for_step, s);
   }
 }
 

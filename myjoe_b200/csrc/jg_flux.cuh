@@ -9,11 +9,23 @@
 
 namespace jg {
 
+// four consecutive doubles in one 32-byte access (p 32-byte aligned): a record of the cell-major
+// arrays is read sector by sector instead of one 8-byte gather per field.  ld4 is for arrays that
+// the kernel does not write
+__device__ __forceinline__ void ld4(double o[4], const double* p) {
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(o[0]), "=d"(o[1]), "=d"(o[2]), "=d"(o[3]) : "l"(p));
+}
+__device__ __forceinline__ void st4(double* p, const double v[4]) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3])
+               : "memory");
+}
+
 // face state; the implicit matrices are templated on the arithmetic type (FP64
 // for the plain form, FP32 for the preconditioner of the mixed form)
 template <typename T>
 struct FStateT {
   T rho, u[3], p, gam;
+  T ig;  // 1 / (gam - 1), formed once on the host: a division less on every side of every face
   T h;  // static enthalpy (the HAENEL flux reads it; the others derive what they need from p, rho)
 };
 using FState = FStateT<double>;
@@ -33,6 +45,7 @@ __device__ __forceinline__ FStateT<T> fstate_as(const FState& s) {
   for (int i = 0; i < 3; i++) o.u[i] = (T)s.u[i];
   o.p = (T)s.p;
   o.gam = (T)s.gam;
+  o.ig = (T)s.ig;
   o.h = (T)s.h;
   return o;
 }
@@ -820,13 +833,30 @@ struct VFace {
   double tau[3];
 };
 
+// RECORDS: the sides' gradients are the state's padded records (32-byte loads), else plain [9] and [3]
+template <bool RECORDS = true>
 __device__ inline void visc_flux(double Fu[3], double& FE, VFace& vf, const VSide& s0, const VSide& s1, double mul,
                                  double mut, double lamOcp, double PrTurb, const double* u_fa, double area,
                                  const double nV[3], double smag, const double sV[3]) {
   double alpha = dot3(nV, sV);
   const double aos = alpha / smag;  // the normal-derivative weight, one division for all terms
-  double g[9];
-  for (int i = 0; i < 9; i++) g[i] = 0.5 * (s0.gu[i] + s1.gu[i]);
+  double g[9], h0[4], h1[4];
+  if (RECORDS) {
+    double a[12], b[12];
+    for (int i = 0; i < 12; i += 4) {
+      ld4(a + i, s0.gu + i);
+      ld4(b + i, s1.gu + i);
+    }
+    ld4(h0, s0.gh);
+    ld4(h1, s1.gh);
+    for (int i = 0; i < 9; i++) g[i] = 0.5 * (a[i] + b[i]);
+  } else {
+    for (int i = 0; i < 9; i++) g[i] = 0.5 * (s0.gu[i] + s1.gu[i]);
+    for (int i = 0; i < 3; i++) {
+      h0[i] = s0.gh[i];
+      h1[i] = s1.gh[i];
+    }
+  }
   double fC[3] = {nV[0] - alpha * sV[0], nV[1] - alpha * sV[1], nV[2] - alpha * sV[2]};
   double div = g[0] + g[4] + g[8];
   double tau[3];
@@ -840,7 +870,7 @@ __device__ inline void visc_flux(double Fu[3], double& FE, VFace& vf, const VSid
   for (int i = 0; i < 3; i++) Fu[i] = -area * tau[i];
   double keff = lamOcp + mut / PrTurb;
   double enth = keff * ((s1.h - s0.h) * aos +
-                        0.5 * ((s0.gh[0] + s1.gh[0]) * fC[0] + (s0.gh[1] + s1.gh[1]) * fC[1] + (s0.gh[2] + s1.gh[2]) * fC[2]));
+                        0.5 * ((h0[0] + h1[0]) * fC[0] + (h0[1] + h1[1]) * fC[1] + (h0[2] + h1[2]) * fC[2]));
   FE = -area * (enth + tau[0] * u_fa[0] + tau[1] * u_fa[1] + tau[2] * u_fa[2]);
   vf.alpha = alpha; vf.smag = smag; vf.area = area; vf.mul = mul; vf.mut = mut; vf.keff = keff; vf.aos = aos;
   for (int i = 0; i < 3; i++) vf.tau[i] = tau[i];

@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(128, MINB) k_flux(Mesh m, Params p, State st, 
         const DevZone z = m.zones[m.bzone[f]];
         const double* bb = &st.bfa[8 * f];
         FState B;
-        B.rho = bb[0]; B.u[0] = bb[1]; B.u[1] = bb[2]; B.u[2] = bb[3]; B.p = bb[4]; B.gam = p.gamma; B.h = bb[6];
+        B.rho = bb[0]; B.u[0] = bb[1]; B.u[1] = bb[2]; B.u[2] = bb[3]; B.p = bb[4]; B.gam = p.gamma; B.ig = p.igm1; B.h = bb[6];
         const FStateT<JT> Bt = fstate_as<JT>(B);
         const JT nVt[3] = {(JT)nV[0], (JT)nV[1], (JT)nV[2]};
         double F[5];
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(128, MINB) k_flux(Mesh m, Params p, State st, 
           v1.h = bb[6]; v1.T = bb[5]; v1.R = p.R; v1.gam = p.gamma;
           v1.gu = v0.gu; v1.gh = v0.gh;
           double sV[3], smag;
-          for (int i = 0; i < 3; i++) sV[i] = m.x_fa[3 * f + i] - m.x_cv[3 * c + i];
+          cell_to_face(m, c, f, sV);
           if (z.kind == JG_BC_WALL) {
             smag = fabs(dot3(sV, nV));  // projected on the wall normal; nVec is used as sVec
             for (int i = 0; i < 3; i++) sV[i] = nV[i];

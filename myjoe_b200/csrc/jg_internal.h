@@ -39,9 +39,11 @@ struct Mesh {
   const double* vol;       // [N]
   const double* x_fa;      // [nfa][3]
   const double* fa_n;      // [nfa][3] area-weighted normal
-  // static face geometry, formed once per mesh (k_face_geo) with the expressions the face loop used
-  // to evaluate per face: fa_u[nfa][4] the unit normal and the area; fa_s[nfa - nfa_b][4] the unit
+  // static geometry records, formed once per mesh (k_cell_geo, k_face_geo) with the expressions the
+  // face loop used to evaluate per face and laid out for its 32-byte loads: xv[N][4] centre and
+  // volume; fa_u[nfa][8] the unit normal, the area, the face centre and a pad; fa_s[nfa - nfa_b][4] the unit
   // vector from cvofa[f][0]'s centre to cvofa[f][1]'s and its length (sVec, smag) of internal faces
+  const double* xv;
   const double* fa_u;
   const double* fa_s;
   const int* cvofa;        // [nfa][2]
@@ -70,21 +72,24 @@ struct Mesh {
   const int* case_of;      // [N] case of each cell (batches)
 };
 
-// Per-case device state.  Primitive record: u,v,w,p,T,h,c,pad.  Boundary
-// record: rho,u,v,w,p,T,h,pad.  Gradients: [N][9] u, [N][3] rho, p, h.
+// Per-case device state.  Primitive record: u,v,w,p,T,h,c,rho (64 bytes: two 32-byte loads give a
+// neighbour's whole state).  Boundary record: rho,u,v,w,p,T,h,pad.  Gradient record (GS doubles,
+// 128 bytes: four loads): u 9, rho 3, p 3, pad; the enthalpy gradient has its own (GHS).
+constexpr int GS = 16, GHS = 4;
 struct State {
   double* q;        // [N][5] conserved (rho, rhou, rhoE)
   double* prim;     // [N][8]
   double* bfa;      // [nfa_b][8]
   double* mul_fa;   // [nfa]
   double* lam_fa;   // [nfa] lambda/cp
-  double* gu;       // [N][9] Euler (second order) gradient of velocity
-  double* guv;      // [N][9] viscous gradient of velocity (may alias gu)
-  double* grho;     // [N][3]
-  double* gp;       // [N][3]
-  double* gh;       // [N][3]
+  double* gu;       // [N][GS] Euler (second order) gradient of velocity, the gradient record's start
+  double* guv;      // [N][GS] viscous gradient of velocity (may alias gu)
+  double* grho;     // gu + 9
+  double* gp;       // gu + 12
+  double* gh;       // [N][GHS]
   double* local_dt; // [N]
   double* rhs;      // [N][5] RHS of calcRhs (rho, rhou, rhoE)
+  double* ff;       // [nfa][8], viscous [nfa][12]: the face fluxes of the split face loop (5x5 path)
   unsigned char* shock_flag;  // [N] AUSMDV shock fix: the cell touches a sonic internal face
   double* jst;                // [N][8] JST: pressure sensor, spectral radius, internal faces, undivided Laplacian[5]
   const unsigned char* jst_bcv;  // [N] JST's BoundaryCV: the cell is the first cell of an internal face
@@ -142,6 +147,7 @@ struct Turb {
 
 struct Params {
   double gamma, R, Pr, PrTurb;
+  double igm1;      // 1 / (gamma - 1) (set with gamma)
   double cp;        // gamma R / (gamma - 1), the enthalpy per kelvin (set with gamma and R)
   double gravity[3];  // GX, GY, GZ of sourceHook; has_gravity: any of them non-zero
   int has_gravity;
@@ -159,8 +165,7 @@ struct Params {
   int fp32;         // matrix + relaxation in FP32
   int turb;         // JG_TURB_*
   // launch shapes (jg_autotune / jg_set_launch_config): the 5x5 face loop (fused: 1, 2 or 4
-  // lanes per cell or JG_FLUX_CL1_3BLK; split: JG_FLUX_SPLIT + lanes per cell of the residual
-  // kernel), and the 5x5 Jacobi sweep's kernel (0: a block per 32-cell slice with a thread per
+  // lanes per cell or JG_FLUX_CL1_3BLK; split: JG_FLUX_SPLIT + 1, 2, 4 or 8, one shape), and the 5x5 Jacobi sweep's kernel (0: a block per 32-cell slice with a thread per
   // block row, 1: a thread per cell)
   int flux_cl;
   int relax_variant;
@@ -192,16 +197,15 @@ void launch_grad(const Mesh& m, const Params& p, State& st, cudaStream_t s);
 void launch_flux(const Mesh& m, const Params& p, State& st, int implicit, int for_step, cudaStream_t s);
 void launch_flux_fused(const Mesh& m, const Params& p, State& st, int for_step, cudaStream_t s);
 void launch_face_sensors(const Mesh& m, const Params& p, State& st, cudaStream_t s);
-void launch_face_geo(const Mesh& m, double* fa_u, double* fa_s, cudaStream_t s);
+void launch_geo(const Mesh& m, double* xv, double* fa_u, double* fa_s, cudaStream_t s);
 // jg_step_host's upload (pack + state + history base) and download (unpack + flags + residuals)
 void launch_state_in(const Mesh& m, const Params& p, State& st, const double* rho, const double* rhou,
                      const double* rhoE, const int* perm, cudaStream_t s);
 void launch_state_out(const Mesh& m, State& st, double* rho, double* rhou, double* rhoE, const int* perm, double* out,
                       int nres, cudaStream_t s);
-// face-loop launch shapes: split (residual kernel with FL lanes per cell + Jacobian kernel)
-// are JG_FLUX_SPLIT + FL; the others are the fused kernel's
+// face-loop launch shapes: split (residual and Jacobian kernels) from JG_FLUX_SPLIT on; the others
+// are the fused kernel's
 inline bool flux_split(const Params& p, const State& st) { return p.flux_cl >= JG_FLUX_SPLIT || st.jac_lag > 1; }
-inline int flux_split_lanes(const Params& p) { return p.flux_cl >= JG_FLUX_SPLIT ? p.flux_cl - JG_FLUX_SPLIT : 4; }
 void launch_resid(const Mesh& m, State& st, int hist_index_from_ctrl, cudaStream_t s);
 // per-case residual history, resid[(idx*ncases + case)*5 + i]
 // per-case L1 residual: RCHUNK-cell chunks counted from each case's first cell

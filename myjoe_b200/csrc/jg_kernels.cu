@@ -47,6 +47,7 @@ __device__ __forceinline__ void state_from_q(const Params& p, const double* q, d
   prim[4] = T;
   prim[5] = p.cp * T;
   prim[6] = sqrt(p.gamma * pp / r);
+  prim[7] = r;
 }
 
 // state errors are recorded per case (a batch keeps going); a frozen case keeps its primitives
@@ -97,10 +98,8 @@ __global__ void k_update_state_x(Mesh m, Params p, State st, const BT* __restric
 __device__ __forceinline__ void face_props(const Mesh& m, const Params& p, State& st, int f) {
   int c0 = m.cvofa[2 * f], c1 = m.cvofa[2 * f + 1];
   double d0[3], d1[3];
-  for (int i = 0; i < 3; i++) {
-    d0[i] = m.x_fa[3 * f + i] - m.x_cv[3 * c0 + i];
-    d1[i] = m.x_fa[3 * f + i] - m.x_cv[3 * c1 + i];
-  }
+  cell_to_face(m, c0, f, d0);
+  cell_to_face(m, c1, f, d1);
   double w0 = sqrt(dot3(d0, d0)), w1 = sqrt(dot3(d1, d1));
   double T = (w1 * st.prim[8 * c0 + 4] + w0 * st.prim[8 * c1 + 4]) / (w0 + w1);
   double mu = mu_law(p, T);
@@ -438,8 +437,10 @@ __global__ void k_grad(Mesh m, Params p, State st, int do_euler, int do_visc, in
                        int separate_guv) {
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.ncv || !st.case_active[m.case_of[c]]) return;  // a frozen case keeps its arrays
-  const double* pc = &st.prim[8 * c];
-  double rc = st.q[5 * c];
+  double pc[8];
+  ld4(pc, &st.prim[(size_t)8 * c]);
+  ld4(pc + 4, &st.prim[(size_t)8 * c + 4]);
+  const double rc = pc[7];
   // raw LSQ sums: diagonal, neighbours (nbocv order), then boundary faces
   double gu[9], gr[3], gpr[3], gh[3];
   int k0 = m.nb_i[c], k1 = m.nb_i[c + 1];
@@ -458,8 +459,10 @@ __global__ void k_grad(Mesh m, Params p, State st, int do_euler, int do_visc, in
   for (int k = k0 + 1; k < k1; k++) {
     int nb = m.nb_v[k];
     double w[3] = {m.lsq[3 * k], m.lsq[3 * k + 1], m.lsq[3 * k + 2]};
-    const double* pn = &st.prim[8 * nb];
-    double rn = st.q[5 * nb];
+    double pn[8];
+    ld4(pn, &st.prim[(size_t)8 * nb]);
+    ld4(pn + 4, &st.prim[(size_t)8 * nb + 4]);
+    const double rn = pn[7];
     for (int i = 0; i < 3; i++) {
       for (int j = 0; j < 3; j++) gu[3 * i + j] += w[j] * pn[i];
       umax[i] = fmax(umax[i], pn[i]);
@@ -561,11 +564,14 @@ __global__ void k_grad(Mesh m, Params p, State st, int do_euler, int do_visc, in
   for (int i = 0; i < 3; i++) lu[i] = (umax[i] - umin[i]) > 1.0e-8;
   if (p.limiter) {
     BjRatio bu[3], br, bp, bh;
+    double xc[4];
+    ld4(xc, &m.xv[(size_t)4 * c]);
     for (int k = m.slot_i[c]; k < m.slot_i[c + 1]; k++) {
       Slot s = m.slots[k];
       if (s.nb < 0) continue;
-      double r0[3];
-      for (int j = 0; j < 3; j++) r0[j] = m.x_fa[3 * s.f + j] - m.x_cv[3 * c + j];
+      double xf[4], r0[3];
+      ld4(xf, &m.fa_u[(size_t)8 * s.f + 4]);
+      for (int j = 0; j < 3; j++) r0[j] = xf[j] - xc[j];
       for (int i = 0; i < 3; i++)
         if (lu[i]) bj_min(bu[i], pc[i], pc[i] + dot3(r0, &gu[3 * i]), umax[i], umin[i], e2u);
       if (lr) bj_min(br, rc, rc + dot3(r0, gr), rmax, rmin, e2r);
@@ -583,19 +589,22 @@ __global__ void k_grad(Mesh m, Params p, State st, int do_euler, int do_visc, in
     if (!lh) ah = 0.0;
   }
   if (do_euler) {
+    double g[GS];
     for (int i = 0; i < 3; i++)
-      for (int j = 0; j < 3; j++) st.gu[9 * c + 3 * i + j] = p.limiter ? gu[3 * i + j] * au[i] : gu[3 * i + j];
+      for (int j = 0; j < 3; j++) g[3 * i + j] = p.limiter ? gu[3 * i + j] * au[i] : gu[3 * i + j];
     for (int j = 0; j < 3; j++) {
-      st.grho[3 * c + j] = p.limiter ? gr[j] * ar : gr[j];
-      st.gp[3 * c + j] = p.limiter ? gpr[j] * ap : gpr[j];
+      g[9 + j] = p.limiter ? gr[j] * ar : gr[j];
+      g[12 + j] = p.limiter ? gpr[j] * ap : gpr[j];
     }
+    g[15] = 0.0;
+    for (int i = 0; i < GS; i += 4) st4(&st.gu[(size_t)GS * c + i], g + i);
   }
   if (do_visc) {
     if (separate_guv || !do_euler) {
       for (int i = 0; i < 3; i++)
-        for (int j = 0; j < 3; j++) st.guv[9 * c + 3 * i + j] = visc_lim_u ? gu[3 * i + j] * au[i] : gu[3 * i + j];
+        for (int j = 0; j < 3; j++) st.guv[(size_t)GS * c + 3 * i + j] = visc_lim_u ? gu[3 * i + j] * au[i] : gu[3 * i + j];
     }
-    for (int j = 0; j < 3; j++) st.gh[3 * c + j] = visc_lim_h ? gh[j] * ah : gh[j];
+    for (int j = 0; j < 3; j++) st.gh[(size_t)GHS * c + j] = visc_lim_h ? gh[j] * ah : gh[j];
   }
 }
 
@@ -954,8 +963,8 @@ __global__ void k_flux_faces(int kind, int n, const double* L, const double* R, 
   int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= n) return;
   FState sl, sr;
-  sl.rho = L[6 * f]; sl.u[0] = L[6 * f + 1]; sl.u[1] = L[6 * f + 2]; sl.u[2] = L[6 * f + 3]; sl.p = L[6 * f + 4]; sl.gam = L[6 * f + 5];
-  sr.rho = R[6 * f]; sr.u[0] = R[6 * f + 1]; sr.u[1] = R[6 * f + 2]; sr.u[2] = R[6 * f + 3]; sr.p = R[6 * f + 4]; sr.gam = R[6 * f + 5];
+  sl.rho = L[6 * f]; sl.u[0] = L[6 * f + 1]; sl.u[1] = L[6 * f + 2]; sl.u[2] = L[6 * f + 3]; sl.p = L[6 * f + 4]; sl.gam = L[6 * f + 5]; sl.ig = 1.0 / (sl.gam - 1.0);
+  sr.rho = R[6 * f]; sr.u[0] = R[6 * f + 1]; sr.u[1] = R[6 * f + 2]; sr.u[2] = R[6 * f + 3]; sr.p = R[6 * f + 4]; sr.gam = R[6 * f + 5]; sr.ig = 1.0 / (sr.gam - 1.0);
   // ideal-gas enthalpy from the state (HAENEL)
   sl.h = sl.gam * sl.p / ((sl.gam - 1.0) * sl.rho);
   sr.h = sr.gam * sr.p / ((sr.gam - 1.0) * sr.rho);
@@ -1068,8 +1077,13 @@ __global__ void k_face_geo(Mesh m, double* fa_u, double* fa_s) {
   if (f >= m.nfa) return;
   const double n[3] = {m.fa_n[3 * f], m.fa_n[3 * f + 1], m.fa_n[3 * f + 2]};
   const double area = sqrt(dot3(n, n));
-  for (int i = 0; i < 3; i++) fa_u[4 * f + i] = n[i] / area;
-  fa_u[4 * f + 3] = area;
+  double* u = &fa_u[8 * (size_t)f];
+  for (int i = 0; i < 3; i++) {
+    u[i] = n[i] / area;
+    u[4 + i] = m.x_fa[3 * f + i];
+  }
+  u[3] = area;
+  u[7] = 0.0;
   if (f >= m.nfa_b) {
     const int c0 = m.cvofa[2 * f], c1 = m.cvofa[2 * f + 1];
     double sV[3];
@@ -1080,7 +1094,14 @@ __global__ void k_face_geo(Mesh m, double* fa_u, double* fa_s) {
     o[3] = smag;
   }
 }
-void launch_face_geo(const Mesh& m, double* fa_u, double* fa_s, cudaStream_t s) {
+__global__ void k_cell_geo(Mesh m, double* xv) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= m.ncv) return;
+  for (int i = 0; i < 3; i++) xv[4 * (size_t)c + i] = m.x_cv[3 * (size_t)c + i];
+  xv[4 * (size_t)c + 3] = m.vol[c];
+}
+void launch_geo(const Mesh& m, double* xv, double* fa_u, double* fa_s, cudaStream_t s) {
+  k_cell_geo<<<grid_for(m.ncv, TB), TB, 0, s>>>(m, xv);
   if (m.nfa > 0) k_face_geo<<<grid_for(m.nfa, TB), TB, 0, s>>>(m, fa_u, fa_s);
 }
 
@@ -1239,7 +1260,7 @@ __global__ void k_visc_faces(int n, const double* S0, const double* S1, const do
   const double u_fa[3] = {ufa[3 * f], ufa[3 * f + 1], ufa[3 * f + 2]};
   double Fu[3], FE;
   VFace vf;
-  visc_flux(Fu, FE, vf, v[0], v[1], mul[f], 0.0, lam[f], 0.9, u_fa, area[f], nV, smag[f], sV);
+  visc_flux<false>(Fu, FE, vf, v[0], v[1], mul[f], 0.0, lam[f], 0.9, u_fa, area[f], nV, smag[f], sV);
   for (int i = 0; i < 3; i++) F[4 * (size_t)f + i] = Fu[i];
   F[4 * (size_t)f + 3] = FE;
   if (A0) {

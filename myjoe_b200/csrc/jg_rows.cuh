@@ -120,23 +120,32 @@ __device__ __forceinline__ void roe_rows(const FStateT<T>& L, const FStateT<T>& 
 template <typename T, typename Emit>
 __device__ __forceinline__ void hllc_rows(const FStateT<T>& L, const FStateT<T>& R, T area, const T nV[3],
                                           Emit&& emit) {
+  // FP64 (D): one reciprocal for the two densities and one for the wave-speed denominator instead
+  // of a division per use (4 instead of 14 a face; k_jac, 300k cells: 239 -> 181 us).  FP32 divides
+  // in a few instructions and keeps the expressions as they were
+  constexpr bool D = sizeof(T) == 8;
+  const T irr = T(1.0) / (L.rho * R.rho), irL = irr * R.rho, irR = irr * L.rho;
   const T unL = dot3(L.u, nV), uLuL = dot3(L.u, L.u);
-  const T cL = sqrt(L.gam * L.p / L.rho);
-  const T eL = (L.gam / (L.gam - T(1.0)) * L.p / L.rho + T(0.5) * uLuL) * L.rho - L.p;
+  const T a2L = D ? L.gam * L.p * irL : L.gam * L.p / L.rho;
+  const T cL = sqrt(a2L);
+  const T eL = D ? L.p * L.ig + T(0.5) * L.rho * uLuL
+                 : (L.gam / (L.gam - T(1.0)) * L.p / L.rho + T(0.5) * uLuL) * L.rho - L.p;
   const T unR = dot3(R.u, nV), uRuR = dot3(R.u, R.u);
-  const T cR = sqrt(R.gam * R.p / R.rho);
-  const T eR = (R.gam / (R.gam - T(1.0)) * R.p / R.rho + T(0.5) * uRuR) * R.rho - R.p;
-  const T Rrho = sqrt(R.rho / L.rho);
+  const T a2R = D ? R.gam * R.p * irR : R.gam * R.p / R.rho;
+  const T cR = sqrt(a2R);
+  const T eR = D ? R.p * R.ig + T(0.5) * R.rho * uRuR
+                 : (R.gam / (R.gam - T(1.0)) * R.p / R.rho + T(0.5) * uRuR) * R.rho - R.p;
+  const T Rrho = sqrt(D ? R.rho * irL : R.rho / L.rho);
   const T tmp = T(1.0) / (T(1.0) + Rrho);
   const T vr[3] = {tmp * (L.u[0] + R.u[0] * Rrho), tmp * (L.u[1] + R.u[1] * Rrho), tmp * (L.u[2] + R.u[2] * Rrho)};
   const T uRoe = dot3(vr, nV);
-  const T gpr = tmp * ((L.gam * L.p / L.rho + T(0.5) * (L.gam - T(1.0)) * uLuL) +
-                       (R.gam * R.p / R.rho + T(0.5) * (R.gam - T(1.0)) * uRuR) * Rrho);
+  const T gpr = tmp * ((a2L + T(0.5) * (L.gam - T(1.0)) * uLuL) + (a2R + T(0.5) * (R.gam - T(1.0)) * uRuR) * Rrho);
   const T cRoe = sqrt(gpr - ((L.gam + R.gam) * T(0.5) - T(1.0)) * T(0.5) * dot3(vr, vr));
   const T sL = fmin(uRoe - cRoe, unL - cL);
   const T sR = fmax(uRoe + cRoe, unR + cR);
-  const T sM = (L.p - R.p - L.rho * unL * (sL - unL) + R.rho * unR * (sR - unR)) /
-               (R.rho * (sR - unR) - L.rho * (sL - unL));
+  const T sMn = L.p - R.p - L.rho * unL * (sL - unL) + R.rho * unR * (sR - unR);
+  const T invrhotld = T(1.0) / (R.rho * (sR - unR) - L.rho * (sL - unL));
+  const T sM = D ? sMn * invrhotld : sMn / (R.rho * (sR - unR) - L.rho * (sL - unL));
   const T pStar = R.rho * (unR - sR) * (unR - sM) + R.p;
   const T gmean = T(0.5) * (L.gam + R.gam);
   if ((sM >= T(0.0) && sL > T(0.0)) || (sM < T(0.0) && sR < T(0.0))) {
@@ -167,7 +176,6 @@ __device__ __forceinline__ void hllc_rows(const FStateT<T>& L, const FStateT<T>&
   T rhouSt[3];
   for (int i = 0; i < 3; i++) rhouSt[i] = (rhoS * uS[i] * sSmu + (pStar - pS_) * nV[i]) * inv;
   const T eSt = (sSmu * eS - pS_ * unS + pStar * sM) * inv;
-  const T invrhotld = T(1.0) / (R.rho * (sR - unR) - L.rho * (sL - unL));
   T dSMdUL[5], dSMdUR[5], dpsdUL[5], dpsdUR[5];
   {
     const T g1 = L.gam - T(1.0);
@@ -198,7 +206,8 @@ __device__ __forceinline__ void hllc_rows(const FStateT<T>& L, const FStateT<T>&
     dpsdO[j] = left ? dpsdUR[j] : dpsdUL[j];
   }
   const T gamma = gmean, gm1 = gamma - T(1.0);
-  const T om = T(1.0) / (sS - sM);
+  const T om = inv;
+  const T HS = D ? (eS + pS_) * (left ? irL : irR) : T(0.0);  // the star side's total enthalpy
   const T SS = sS, SM = sM;
 #pragma unroll
   for (int i = 0; i < 5; i++) {
@@ -221,10 +230,11 @@ __device__ __forceinline__ void hllc_rows(const FStateT<T>& L, const FStateT<T>&
       as[4] = -gm1 * nV[r] + nV[r] * dpsdS[4] + rhouSt[r] * dSMdS[4];
       for (int j = 0; j < 5; j++) ao[j] = om * (nV[r] * dpsdO[j] + rhouSt[r] * dSMdO[j]);
     } else {
-      as[0] = qS * (eS + pS_) / rhoS - qS * psiS * (gamma - T(1.0)) / T(2.0) + SM * dpsdS[0] +
+      as[0] = (D ? qS * HS : qS * (eS + pS_) / rhoS) - qS * psiS * (gamma - T(1.0)) / T(2.0) + SM * dpsdS[0] +
               (pStar + eSt) * dSMdS[0];
       for (int k = 0; k < 3; k++)
-        as[1 + k] = -nV[k] * (eS + pS_) / rhoS + gm1 * uS[k] * qS + SM * dpsdS[1 + k] + (pStar + eSt) * dSMdS[1 + k];
+        as[1 + k] = (D ? -nV[k] * HS : -nV[k] * (eS + pS_) / rhoS) + gm1 * uS[k] * qS + SM * dpsdS[1 + k] +
+                    (pStar + eSt) * dSMdS[1 + k];
       as[4] = SS - qS * gamma + SM * dpsdS[4] + (pStar + eSt) * dSMdS[4];
       for (int j = 0; j < 5; j++) ao[j] = om * (dpsdO[j] * SM + (pStar + eSt) * dSMdO[j]);
     }

@@ -157,6 +157,7 @@ void launch_sweep(const Mesh& m, const State& st, int grid, const BT* xin, BT* x
     static const int fit_wide = resident_blocks(wide, T), fit_mid = resident_blocks(mid, T);
     kernel = grid <= fit_wide ? wide : grid <= fit_mid ? mid : narrow;
   }
+  if (first) kernel = narrow;  // no matrix rows to request: Dinv b
   launch_pass(kernel, grid, T, after_pass, s, m, st, xin, xout, (int)first, color, slices, nullptr, nullptr, nullptr);
 }
 
