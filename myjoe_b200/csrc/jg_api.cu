@@ -60,8 +60,10 @@ struct jg_case {
   size_t eltsz = 8;   // matrix element size
   size_t ell_elems = 0;
   int hist_cap = 0;
-  double* d_tmp = nullptr;  // BiCGSTAB work vectors (9 x 5N) + partials
-  double* d_red = nullptr;
+  double* d_tmp = nullptr;  // BiCGSTAB work vectors (8 x 5N)
+  double* d_red = nullptr;  // its reductions' partial sums and scalars
+  int* bicg_flag = nullptr;  // page-locked: iteration count and stop flag of the running solve
+  cudaEvent_t bicg_ev[2] = {nullptr, nullptr};
   cudaGraphExec_t graph = nullptr;
   int graph_sweeps = -1;
   int primed = 0;           // state + BC computed since the last set_state
@@ -280,7 +282,7 @@ static Params make_params(const jg_params& q) {
   p.under_relax = q.under_relax;
   p.viscous = q.mu_ref > 0.0;
   p.fp32 = q.precision == JG_PREC_MIXED;
-  p.flux_cl = JG_FLUX_SPLIT + 4;  // the split face loop, 4 lanes per cell in the residual
+  p.flux_cl = JG_FLUX_SPLIT + 4;  // the split face loop
   p.relax_variant = 0;
   p.grad_scheme = q.grad_scheme;
   p.ausm_type = q.ausm_type;
@@ -374,6 +376,9 @@ int jg_destroy(jg_case_t* h) {
   if (h->st.ev_fork) cudaEventDestroy(h->st.ev_fork);
   if (h->st.ev_join) cudaEventDestroy(h->st.ev_join);
   if (h->hpin) cudaFreeHost(h->hpin);
+  if (h->bicg_flag) cudaFreeHost(h->bicg_flag);
+  for (cudaEvent_t e : h->bicg_ev)
+    if (e) cudaEventDestroy(e);
   if (h->st.ev_pre) cudaEventDestroy(h->st.ev_pre);
   if (h->st.ev_dt) cudaEventDestroy(h->st.ev_dt);
   if (h->st.ev_res) cudaEventDestroy(h->st.ev_res);
@@ -1422,83 +1427,36 @@ int jg_get_gradients(jg_case_t* h, double* grad_u, double* grad_rho, double* gra
   return JG_OK;
 }
 
-// partial-sum buffer of the BiCGSTAB reductions: launch_dot uses <= 1024
-// blocks, launch_resmax one per 256 cells; the last 16 entries hold scalars
-static size_t red_size(int N) { return (size_t)std::max(1024, grid_for(N, 256)) + 16; }
-
-// BiCGSTAB with the block-diagonal preconditioner, solveCvVectorR5Bcgstab
-// (UgpWithCv.cpp:2660-2876); operates on [5][N] vectors, phi in/out in d_tmp.
+// BiCGSTAB with the block-diagonal or the line preconditioner (jg_bicgstab.cu); operates on [5][N]
+// vectors, phi in/out.  The host enqueues one iteration ahead of the one whose stop flag it reads
+// (a device kernel writes it into page-locked memory); the iteration enqueued past the stop does
+// nothing.
 static int bcgstab(jg_case* h, double* phi, const double* rhs, double zeroAbs, double zeroRel, int maxiter, int* iters,
                    bool lines = false) {
-  const int N = h->ncv;
-  const long n5 = 5L * N;
-  if (!h->d_tmp) {
-    RC(dmalloc(h, &h->d_tmp, 8 * (size_t)n5));
-    RC(dmalloc(h, &h->d_red, red_size(N)));
-  }
-  double *res = h->d_tmp, *res0 = res + n5, *p = res0 + n5, *v = p + n5, *t = v + n5, *s = t + n5, *phat = s + n5,
-         *shat = phat + n5;
-  double* part = h->d_red;
-  double* scal = h->d_red + red_size(N) - 16;
+  const size_t n5 = 5 * (size_t)h->ncv;
+  if (!h->d_tmp) RC(dmalloc(h, &h->d_tmp, 8 * n5));
+  if (!h->d_red) RC(dmalloc(h, &h->d_red, 2048 + 16));
+  if (!h->bicg_flag) CK(cudaHostAlloc(&h->bicg_flag, 2 * sizeof(int), cudaHostAllocDefault));
+  for (cudaEvent_t& e : h->bicg_ev)
+    if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  double* w = h->d_tmp;
+  Bicg q{phi, w, w + n5, w + 2 * n5, w + 3 * n5, w + 4 * n5, w + 5 * n5, w + 6 * n5, w + 7 * n5, h->d_red,
+         h->d_red + 2048, rhs, zeroAbs, zeroRel, maxiter, h->bicg_flag};
   cudaStream_t S = h->stream;
-  auto dot = [&](const double* a, const double* b, double& out) -> int {
-    launch_dot((int)n5, a, b, part, scal, S);
+  h->bicg_flag[0] = h->bicg_flag[1] = 0;
+  CK(cudaMemsetAsync(q.p, 0, 2 * n5 * sizeof(double), S));  // p and v
+  if (lines) launch_line_factor(h->m, h->st, h->lines, S);  // the lines' elimination, once per solve
+  launch_bicg_start(h->m, h->st, q, S);
+  volatile int* flag = h->bicg_flag;
+  for (int k = 0;; k++) {
+    launch_bicg_iteration(h->m, h->st, q, lines ? &h->lines : nullptr, S);
     CKL();
-    CK(cudaMemcpyAsync(&out, scal, sizeof(double), cudaMemcpyDeviceToHost, S));
-    CK(cudaStreamSynchronize(S));
-    return JG_OK;
-  };
-  auto resmax = [&](const double* r, double& out) -> int {
-    launch_resmax(h->m, h->st, r, part, scal, S);
-    CKL();
-    CK(cudaMemcpyAsync(&out, scal, sizeof(double), cudaMemcpyDeviceToHost, S));
-    CK(cudaStreamSynchronize(S));
-    return JG_OK;
-  };
-  CK(cudaMemsetAsync(p, 0, n5 * sizeof(double), S));
-  CK(cudaMemsetAsync(v, 0, n5 * sizeof(double), S));
-  // the preconditioner: block diagonal, or line-implicit (the lines' elimination once per solve)
-  if (lines) launch_line_factor(h->m, h->st, h->lines, S);
-  auto precond = [&](const double* x, double* y) {
-    if (lines) launch_line_precond(h->m, h->st, h->lines, x, y, S);
-    else launch_precond(h->m, h->st, x, y, S);
-  };
-  double rho = 1.0, alpha = 1.0, omega = 1.0;
-  launch_spmv(h->m, h->st, phi, res, S);
-  launch_lin3(n5, res, 1.0, rhs, -1.0, res, 0.0, nullptr, S);
-  CK(cudaMemcpyAsync(res0, res, n5 * sizeof(double), cudaMemcpyDeviceToDevice, S));
-  double res0_max = 0.0, res_max = 0.0;
-  RC(resmax(res, res0_max));
-  int iter = 0, done = 0;
-  while (!done) {
-    iter++;
-    double rho_prime = -omega * rho;
-    RC(dot(res, res0, rho));
-    if (fabs(rho_prime) < 1.0E-20) rho_prime = 1.0E-20;
-    double beta = alpha * rho / rho_prime;
-    // p = res - beta*(p - omega*v)
-    launch_lin3(n5, p, 1.0, res, -beta, p, beta * omega, v, S);
-    precond(p, phat);
-    launch_spmv(h->m, h->st, phat, v, S);
-    double gamma;
-    RC(dot(v, res0, gamma));
-    if (fabs(gamma) < 1.0E-20) gamma = 1.0E-20;
-    alpha = rho / gamma;
-    launch_lin3(n5, s, 1.0, res, -alpha, v, 0.0, nullptr, S);
-    precond(s, shat);
-    launch_spmv(h->m, h->st, shat, t, S);
-    double st_, tt_;
-    RC(dot(s, t, st_));
-    RC(dot(t, t, tt_));
-    omega = st_ / (tt_ + 1.0E-20);
-    launch_lin3(n5, phi, 1.0, phi, alpha, phat, omega, shat, S);
-    launch_spmv(h->m, h->st, phi, res, S);
-    launch_lin3(n5, res, 1.0, rhs, -1.0, res, 0.0, nullptr, S);
-    RC(resmax(res, res_max));
-    if ((res_max <= zeroAbs) || (res_max / (res0_max + 1.0E-12) <= zeroRel)) done = 1;
-    else if (iter > maxiter) done = 2;
+    CK(cudaEventRecord(h->bicg_ev[k % 2], S));
+    if (k == 0) continue;
+    CK(cudaEventSynchronize(h->bicg_ev[(k - 1) % 2]));
+    if (flag[1]) break;
   }
-  if (iters) *iters = iter;
+  if (iters) *iters = flag[0];  // the iteration enqueued past the stop left the count as it was
   return JG_OK;
 }
 
@@ -1524,10 +1482,6 @@ int jg_solve_lin_sys(jg_case_t* h, double* dq, const double* A, const double* rh
   switch (h->hp.lin_solver) {
     case JG_LS_BCGSTAB:
     case JG_LS_BCGSTAB_LINELET: {
-      if (!h->d_tmp) {
-        RC(dmalloc(h, &h->d_tmp, 8 * 5 * (size_t)N));
-        RC(dmalloc(h, &h->d_red, red_size(N)));
-      }
       double* phi = (double*)h->st.x0;
       double* b = (double*)h->st.x1;
       std::vector<double> soa;
@@ -2190,7 +2144,7 @@ extern "C" int jg_autotune(jg_case_t* h, int trials, int* flux_cl, int* relax_va
     State st = h->st;
     st.jac_lag = 1;
     // ms[0..2]: fused, 1, 2, 4 lanes per cell; ms[5]: fused, one lane with three blocks per SM;
-    // ms[6..9]: split, residual with 1, 2, 4, 8 lanes per cell.  A lagged handle runs split.
+    // ms[6..9]: split (one shape under four names).  A lagged handle runs split.
     const int cls[8] = {1, 2, 4, JG_FLUX_CL1_3BLK, JG_FLUX_SPLIT + 1, JG_FLUX_SPLIT + 2, JG_FLUX_SPLIT + 4,
                         JG_FLUX_SPLIT + 8};
     const int slot[8] = {0, 1, 2, 5, 6, 7, 8, 9};

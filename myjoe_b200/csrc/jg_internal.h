@@ -220,13 +220,7 @@ void launch_sgs(const Mesh& m, const Params& p, State& st, int sweeps, cudaStrea
 void launch_dq_from_x(const Mesh& m, const Params& p, State& st, const void* x, cudaStream_t s);
 void launch_lusgs(const Mesh& m, const Params& p, State& st, cudaStream_t s);
 void launch_dinv(const Mesh& m, const Params& p, State& st, cudaStream_t s);
-// BiCGSTAB building blocks (FP64)
-void launch_spmv(const Mesh& m, const State& st, const double* x, double* y, cudaStream_t s);
 void launch_precond(const Mesh& m, const State& st, const double* x, double* y, cudaStream_t s);
-void launch_dot(int n, const double* a, const double* b, double* partial, double* out, cudaStream_t s);
-void launch_resmax(const Mesh& m, const State& st, const double* r, double* partial, double* out, cudaStream_t s);
-void launch_lin3(long n, double* out, double a, const double* x, double b, const double* y, double c, const double* z,
-                 cudaStream_t s);
 void launch_flux_faces(int kind, int n, const double* L, const double* R, const double* area, const double* nvec,
                        double* F, double* AL, double* AR, cudaStream_t s);
 
@@ -300,6 +294,19 @@ void launch_aos_to_soa5(int n, const double* aos, double* soa, cudaStream_t s);
 // the result is in st.x0 (odd sweeps) or st.x1 (even)
 void launch_line_relax(const Mesh& m, const Params& p, State& st, const Lines& L, int bs, int sweeps,
                        cudaStream_t s);
+
+// one BiCGSTAB solve (jg_bicgstab.cu): vectors [5][N], the partial sums of the reductions (2,048
+// doubles), 16 doubles of device scalars, and the host's view of the iteration count and the stop
+// flag (page-locked, two ints)
+struct Bicg {
+  double *phi, *res, *res0, *p, *v, *t, *s, *phat, *shat, *part, *sc;
+  const double* rhs;
+  double zabs, zrel;
+  int maxiter;
+  volatile int* flag;
+};
+void launch_bicg_start(const Mesh& m, const State& st, const Bicg& q, cudaStream_t s);
+void launch_bicg_iteration(const Mesh& m, const State& st, const Bicg& q, const Lines* lines, cudaStream_t s);
 
 // A mesh in jg_mesh's layout whose arrays the struct owns (concatenated
 // batches, renumbered cases); bind() points m at the vectors.

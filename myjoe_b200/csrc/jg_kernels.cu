@@ -854,34 +854,7 @@ __global__ void k_lusgs2(Mesh m, State st, const double* xs, double* x1) {
   }
 }
 
-// ---------------------------------------------------------------------------
-// BiCGSTAB building blocks (solveCvVectorR5Bcgstab, UgpWithCv.cpp:2660-2876), FP64, [5][N]
-// ---------------------------------------------------------------------------
-__global__ void k_spmv(Mesh m, State st, const double* x, double* y) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= m.ncv) return;
-  const int N = m.ncv;
-  const double* D = (const double*)st.D;
-  const double* O = (const double*)st.O;
-  double acc[5];
-  for (int i = 0; i < 5; i++) {
-    double s = 0.0;
-    for (int k = 0; k < 5; k++) s += D[(size_t)(5 * i + k) * N + c] * x[(size_t)k * N + c];
-    acc[i] = s;
-  }
-  int slice = c / SLICE, lane = c % SLICE;
-  for (int j = m.ell_off[slice]; j < m.ell_off[slice + 1]; j++) {
-    int nb = m.ell_nb[(size_t)j * SLICE + lane];
-    const double* Ob = O + (size_t)j * 25 * SLICE + lane;
-    for (int i = 0; i < 5; i++) {
-      double s = 0.0;
-      for (int k = 0; k < 5; k++) s += Ob[(5 * i + k) * SLICE] * x[(size_t)k * N + nb];
-      acc[i] += s;
-    }
-  }
-  for (int i = 0; i < 5; i++) y[(size_t)i * N + c] = acc[i];
-}
-
+// y = Dinv x, [5][N]
 __global__ void k_precond(Mesh m, State st, const double* x, double* y) {
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.ncv) return;
@@ -894,67 +867,6 @@ __global__ void k_precond(Mesh m, State st, const double* x, double* y) {
     for (int k = 0; k < 5; k++) s += Di[(size_t)(5 * i + k) * N + c] * xv[k];
     y[(size_t)i * N + c] = s;
   }
-}
-
-__global__ void k_dot_partial(int n, const double* a, const double* b, double* partial) {
-  __shared__ double s[256];
-  double v = 0.0;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) v += a[i] * b[i];
-  s[threadIdx.x] = v;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) s[threadIdx.x] += s[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) partial[blockIdx.x] = s[0];
-}
-
-__global__ void k_sum_final(int nblk, const double* partial, double* out, int is_max) {
-  __shared__ double s[256];
-  double v = 0.0;
-  for (int i = threadIdx.x; i < nblk; i += blockDim.x) v = is_max ? fmax(v, partial[i]) : v + partial[i];
-  s[threadIdx.x] = v;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) s[threadIdx.x] = is_max ? fmax(s[threadIdx.x], s[threadIdx.x + w]) : s[threadIdx.x] + s[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *out = s[0];
-}
-
-// max over cells of |D^-1 r| (the reference's preconditioned residual norm)
-__global__ void k_resmax_partial(Mesh m, State st, const double* r, double* partial) {
-  __shared__ double s[256];
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  double v = 0.0;
-  if (c < m.ncv) {
-    const int N = m.ncv;
-    const double* Di = (const double*)st.Dinv;
-    double rv[5];
-    for (int k = 0; k < 5; k++) rv[k] = r[(size_t)k * N + c];
-    for (int i = 0; i < 5; i++) {
-      double t = 0.0;
-      for (int k = 0; k < 5; k++) t += Di[(size_t)(5 * i + k) * N + c] * rv[k];
-      v = fmax(v, fabs(t));
-    }
-  }
-  s[threadIdx.x] = v;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) s[threadIdx.x] = fmax(s[threadIdx.x], s[threadIdx.x + w]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) partial[blockIdx.x] = s[0];
-}
-
-// out = a*x + b*y + c*z (z may be null); out may alias x, y or z
-__global__ void k_lin3(long n, double* out, double a, const double* x, double b, const double* y, double c,
-                       const double* z) {
-  long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double v = a * x[i] + b * y[i];
-  if (z) v += c * z[i];
-  out[i] = v;
 }
 
 // batched face fluxes (per-face parity entry point)
@@ -1206,26 +1118,8 @@ void launch_lusgs(const Mesh& m, const Params& p, State& st, cudaStream_t s) {
   k_jacobi<double><<<grid_for(m.ncv, TB), TB, 0, s>>>(m, st, (const double*)st.x1, (double*)st.x0, 1);
   k_lusgs2<<<grid_for(m.ncv, TB), TB, 0, s>>>(m, st, (const double*)st.x0, (double*)st.x1);
 }
-void launch_spmv(const Mesh& m, const State& st, const double* x, double* y, cudaStream_t s) {
-  k_spmv<<<grid_for(m.ncv, TB), TB, 0, s>>>(m, st, x, y);
-}
 void launch_precond(const Mesh& m, const State& st, const double* x, double* y, cudaStream_t s) {
   k_precond<<<grid_for(m.ncv, TB), TB, 0, s>>>(m, st, x, y);
-}
-void launch_dot(int n, const double* a, const double* b, double* partial, double* out, cudaStream_t s) {
-  int nb = grid_for(n, 256);
-  if (nb > 1024) nb = 1024;
-  k_dot_partial<<<nb, 256, 0, s>>>(n, a, b, partial);
-  k_sum_final<<<1, 256, 0, s>>>(nb, partial, out, 0);
-}
-void launch_resmax(const Mesh& m, const State& st, const double* r, double* partial, double* out, cudaStream_t s) {
-  int nb = grid_for(m.ncv, 256);
-  k_resmax_partial<<<nb, 256, 0, s>>>(m, st, r, partial);
-  k_sum_final<<<1, 256, 0, s>>>(nb, partial, out, 1);
-}
-void launch_lin3(long n, double* out, double a, const double* x, double b, const double* y, double c, const double* z,
-                 cudaStream_t s) {
-  k_lin3<<<grid_for(n, 256), 256, 0, s>>>(n, out, a, x, b, y, c, z);
 }
 void launch_flux_faces(int kind, int n, const double* L, const double* R, const double* area, const double* nvec,
                        double* F, double* AL, double* AR, cudaStream_t s) {
