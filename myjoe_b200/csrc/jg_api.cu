@@ -783,17 +783,16 @@ static int build(jg_case* h, const jg_mesh* mesh, const jg_params* q) {
       RC(dmalloc(h, &L.up, 25 * nc));
       RC(dmalloc(h, &L.v, 5 * nc));
     } else {
-      // the line cells, and per cell the ELL rows of its couplings off the line and per slice their end
-      std::vector<uint8_t> on_line(N, 0);
+      // per cell its line position and the number of its couplings off the line, per slice their last ELL row
+      std::vector<int> line_pos(N, -1);
       std::vector<int> off_end(nslices);
-      for (int k = 0; k < L.nlines; k++)
-        for (int i = off[k]; i < off[k + 1]; i++) on_line[cv[i]] = 1;
+      for (int i = 0; i < off[L.nlines]; i++) line_pos[cv[i]] = i;
       for (int sl = 0; sl < nslices; sl++) {
         int w = 0;
         for (int c = sl * SLICE; c < std::min(N, (sl + 1) * SLICE); c++) w = std::max(w, noff[c]);
         off_end[sl] = h->ell_off[sl] + w;
       }
-      RC(upload(h, &L.on_line, on_line.data(), on_line.size()));
+      RC(upload(h, &L.line_pos, line_pos.data(), line_pos.size()));
       RC(upload(h, &L.noff, noff.data(), noff.size()));
       RC(upload(h, &L.off_end, off_end.data(), off_end.size()));
       RC(dmalloc_bytes(h, &L.binv, (size_t)bs * bs * nc * h->eltsz));
@@ -915,7 +914,7 @@ static size_t footprint(const jg_mesh* mesh, const jg_params* q, const std::vect
     if (q->lin_solver == JG_LS_BCGSTAB_LINELET)
       b += 3 * alloc_round(25 * nc * d) + alloc_round(5 * nc * d);
     else
-      b += alloc_round(N) + alloc_round(N * i) + alloc_round(nslices * i) + 3 * alloc_round(b2 * nc * e) +
+      b += 2 * alloc_round(N * i) + alloc_round(nslices * i) + 3 * alloc_round(b2 * nc * e) +
            alloc_round(bs * nc * e);
   }
   return b;
@@ -1204,6 +1203,7 @@ static int check_err_flags(jg_case* h, bool all_cases = false, const double* dre
   if (e) {
     CK(cudaMemsetAsync(h->st.err, 0, sizeof(int), h->stream));
     if (e & 2) return set_err(JG_ERR_ARG, "unrecognised boundary condition");
+    if (e & 8) return set_err(JG_ERR_CUDA, "line substitutions: an asynchronous copy did not complete");
     return set_err(JG_ERR_STATE, "non-physical state (flags %d): negative density/pressure or NaN residual", e);
   }
   return JG_OK;

@@ -165,8 +165,9 @@ struct Params {
   int fp32;         // matrix + relaxation in FP32
   int turb;         // JG_TURB_*
   // launch shapes (jg_autotune / jg_set_launch_config): the 5x5 face loop (fused: 1, 2 or 4
-  // lanes per cell or JG_FLUX_CL1_3BLK; split: JG_FLUX_SPLIT + 1, 2, 4 or 8, one shape), and the 5x5 Jacobi sweep's kernel (0: a block per 32-cell slice with a thread per
-  // block row, 1: a thread per cell)
+  // lanes per cell or JG_FLUX_CL1_3BLK; split: JG_FLUX_SPLIT + 1, 2, 4 or 8, one shape), and the
+  // 5x5 Jacobi sweep's kernel (0: a block per 32-cell slice with a thread per block row, 1: a
+  // thread per cell)
   int flux_cl;
   int relax_variant;
   int grad_scheme;  // JG_GRAD_*
@@ -271,7 +272,7 @@ struct Lines {
   double* up;      // [off[nlines]][25] (position 0 of a line unused)
   double* v;       // [off[nlines]][5]
   // LINE relaxation (B x B blocks in the matrix precision)
-  const uint8_t* on_line;     // [N] 1 on the cells of the lines
+  const int* line_pos;        // [N] the cell's position in cv, -1 off the lines
   const int* noff;            // [N] couplings of the cell that are not to its line neighbours: its first ELL columns
   const int* off_end;         // [nslices] one past the last ELL row holding such a coupling of a cell of the slice
   void* binv;      // [off[nlines]][B*B]

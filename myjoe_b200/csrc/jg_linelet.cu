@@ -23,6 +23,7 @@
 // the 5 rows (substitutions) of one block step.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "jg_internal.h"
@@ -280,8 +281,8 @@ void launch_line_precond(const Mesh& m, const State& st, const Lines& L, const d
 // block-tridiagonal part of A along the lines (the block diagonal elsewhere):
 //   k_sweep (LINE): per cell r = b - sum of the off-diagonal blocks that are not
 //                 a line coupling times x; off the lines x' = Dinv r, on the
-//                 lines r is left in x' for
-//   k_lsolve:     the block Thomas substitutions of each line, in place.
+//                 lines r is left in line order for
+//   k_lsolve:     the block Thomas substitutions of each line, into x'.
 // k_lfactor computes the line factors once per step from D and the ELL
 // blocks, in FP64 arithmetic, and stores them in BT.  (The LINE relaxation has
 // no reference counterpart; the reference's own line solver, BCGSTAB_LINELET,
@@ -410,89 +411,166 @@ __global__ void __launch_bounds__(32 * LW) k_lfactor(Mesh m, State st, Lines L) 
   }
 }
 
-// x (cells of a line) = T_line^-1 r, r read from x.  Four lines per warp, eight lanes per line
-// (lanes < B of a group hold the rows of its blocks): the chain along a line is serial, so a
-// warp's lines advance together, each step costing one warp's latency for four lines.  The
-// operands of the steps (a matrix row, the cell id, the right-hand side) do not depend on the
-// chain: they are loaded LK steps at a time into one of two register sets, the next chunk's
-// loads issued before the current chunk's steps compute (and its cell ids a chunk earlier), so a
-// chunk's memory latency runs under the previous chunk's arithmetic.  The shuffles run on every lane; a group past the end of its
-// line only skips the update.
-constexpr int LK = 4;
+// Bulk copies from global to shared memory (the copy engine, one instruction a run of positions) and
+// the barrier a stage of them completes on.  A copy starts and ends on 16-byte boundaries, so one of
+// `len` bytes at p takes the aligned bytes around it; shift16(p) is where p then lies.
+__device__ __forceinline__ unsigned sh_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ unsigned shift16(const void* p) { return (unsigned)((uintptr_t)p & 15); }
+__device__ __forceinline__ unsigned bulk_bytes(const void* p, unsigned len) { return (shift16(p) + len + 15) & ~15u; }
+__device__ __forceinline__ void bulk_copy(void* dst, const void* p, unsigned len, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   sh_addr(dst)),
+               "l"((const char*)p - shift16(p)), "r"(bulk_bytes(p, len)), "r"(sh_addr(bar))
+               : "memory");
+}
+__device__ __forceinline__ void bar_expect(uint64_t* bar, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sh_addr(bar)), "r"(bytes) : "memory");
+}
+// false if the barrier's phase has not completed after a bounded number of tries
+__device__ __forceinline__ bool bar_wait(uint64_t* bar, unsigned parity) {
+  for (int i = 0; i < 1 << 20; i++) {
+    unsigned ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(sh_addr(bar)), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+
 constexpr int LG = 8;         // lanes per line
 constexpr int LPW = 32 / LG;  // lines per warp
 
+// a stage holds LK positions of each of a warp's lines: two blocks and a vector a position, and room
+// for the bytes an unaligned start or end adds
 template <typename BT, int B>
-__global__ void __launch_bounds__(32 * LW) k_lsolve(Mesh m, Lines L, BT* __restrict__ x) {
+struct LineRing {
+  static constexpr int LK = 32 / sizeof(BT), LS = 3;
+  static constexpr int BLK = LK * B * B * sizeof(BT) + 16, VEC = LK * B * sizeof(BT) + 16;
+  static constexpr int LINE = 2 * BLK + VEC;
+};
+
+// a row of a block (B elements), in 16- or 8-byte loads where rows are so aligned
+template <typename BT, int B>
+__device__ __forceinline__ void load_row(BT o[B], const BT* p) {
+  if constexpr (B == 6) {
+    using V = typename std::conditional<sizeof(BT) == 8, double2, float2>::type;
+#pragma unroll
+    for (int q = 0; q < B; q += 2) {
+      const V v = *reinterpret_cast<const V*>(p + q);
+      o[q] = v.x;
+      o[q + 1] = v.y;
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < B; q++) o[q] = p[q];
+  }
+}
+
+// x (cells of a line) = T_line^-1 r, r in line order in L.bv (the pass before left it there).  Four
+// lines per warp, eight lanes per line (lanes < B of a group hold the rows of its blocks): the chain
+// along a line is serial, so a warp's lines advance together.  The operands of the steps do not
+// depend on the chain and lie in line order, so the copy engine brings them LS - 1 stages ahead
+// into shared memory and a step's instructions are its row loads, shuffles and multiply-adds: with
+// about one warp per scheduler it is the instructions of a step that cost.  2,048 lines of 20 to 80
+// cells, register double-buffering before -> now: 6x6 FP64 44 -> 39 us, FP32 36 -> 25; 7x7 FP32 32 -> 21.
+// The shuffles run on every lane; a group past the end of its line only skips the update.  A stage
+// that never completes (err gets 8) ends the pass, not the kernel's copies.
+template <typename BT, int B>
+__global__ void __launch_bounds__(32) k_lsolve(Mesh m, Lines L, BT* __restrict__ x, int* err) {
   static_assert(B <= LG, "a line's rows fit its lane group");
-  constexpr int BB = B * B;
-  constexpr int K = sizeof(BT) * B > 48 ? LK / 2 : LK;  // steps per chunk (FP64 7x7: two register sets fit at LK / 2)
-  const int w = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int r = lane % LG;
-  const int line = (blockIdx.x * LW + w) * LPW + lane / LG;
+  using R = LineRing<BT, B>;
+  constexpr int BB = B * B, K = R::LK, S = R::LS;
+  __shared__ __align__(16) unsigned char ring[S][LPW][R::LINE];
+  __shared__ uint64_t bars[S];
+  const int lane = threadIdx.x, r = lane % LG, g = lane / LG;
+  const int line = blockIdx.x * LPW + g;
   const bool has = line < L.nlines;
   const int p0 = has ? L.off[line] : 0, n = has ? L.off[line + 1] - p0 : 0;
   const bool row = has && r < B;
   const int rr = r < B ? r : 0;  // lanes past the rows mirror row 0 and never store
+  if (lane == 0) {
+    for (int s = 0; s < S; s++)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sh_addr(&bars[s])), "r"(LPW) : "memory");
+    asm volatile("fence.proxy.async;" ::: "memory");
+  }
+  __syncwarp();
   int nmax = n;
   for (int o = LG; o < 32; o *= 2) nmax = max(nmax, __shfl_xor_sync(0xffffffffu, nmax, o));
-  if (nmax == 0) return;  // the whole warp (no line of its own)
   const size_t N = m.ncv;
   const BT* Linv = (const BT*)L.binv;
   const BT* Llow = (const BT*)L.blow;
   const BT* Lup = (const BT*)L.bup;
   BT* Lv = (BT*)L.bv;
-  // forward: v_0 = r_0, v_i = r_i - low_i v_{i-1}
-  BT v = has ? x[rr * N + L.cv[p0]] : BT(0);
-  if (row) Lv[(size_t)p0 * B + r] = v;
-  // the operands of steps i0 .. i0 + K - 1 (past the line's end: zeros), called chunk after
-  // chunk; their cell ids were loaded by the call before, and this call loads the next chunk's
-  int cn[K];
-#pragma unroll
-  for (int t = 0; t < K; t++) cn[t] = (1 + t < n) ? L.cv[p0 + 1 + t] : 0;
-  auto load_fwd = [&](int i0, BT(&mi)[K][B], BT(&xi)[K]) {
-#pragma unroll
-    for (int t = 0; t < K; t++) {
-      const int i = i0 + t;
-      if (i < n) {
-#pragma unroll
-        for (int q = 0; q < B; q++) mi[t][q] = Llow[(size_t)(p0 + i) * BB + B * rr + q];
-        xi[t] = x[rr * N + cn[t]];
-      } else {
-#pragma unroll
-        for (int q = 0; q < B; q++) mi[t][q] = BT(0);
-        xi[t] = BT(0);
-      }
+  const int chunks = (nmax - 1 + K - 1) / K;  // steps 0 .. nmax - 2 of each pass
+  bool ok = true;
+  // forward: v_0 = r_0, v_i = r_i - low_i v_{i-1}; step j is position j + 1.  Stage q % S holds the
+  // q-th chunk asked for, forward chunks first
+  auto ask_fwd = [&](int c) {
+    if (r != 0 || c >= chunks) return;
+    const int i = c * K + 1, cnt = min(K, n - i);
+    uint64_t* bar = &bars[c % S];
+    if (cnt <= 0) {
+      bar_expect(bar, 0);
+      return;
     }
-#pragma unroll
-    for (int t = 0; t < K; t++) cn[t] = (i0 + K + t < n) ? L.cv[p0 + i0 + K + t] : 0;
+    unsigned char* d = ring[c % S][g];
+    const BT *lo = Llow + (size_t)(p0 + i) * BB, *rv = Lv + (size_t)(p0 + i) * B;
+    const unsigned lb = cnt * BB * sizeof(BT), vb = cnt * B * sizeof(BT);
+    bar_expect(bar, bulk_bytes(lo, lb) + bulk_bytes(rv, vb));
+    bulk_copy(d, lo, lb, bar);
+    bulk_copy(d + 2 * R::BLK, rv, vb, bar);
   };
-  auto step_fwd = [&](int i0, const BT(&mi)[K][B], const BT(&xi)[K]) {
+  for (int c = 0; c < S - 1; c++) ask_fwd(c);
+  BT v = has ? Lv[(size_t)p0 * B + rr] : BT(0);
+  for (int c = 0; c < chunks; c++) {
+    ok = bar_wait(&bars[c % S], (c / S) & 1) && ok;
+    const int i0 = c * K + 1;
+    const unsigned char* d = ring[c % S][g];
+    const BT* lo = reinterpret_cast<const BT*>(d + shift16(Llow + (size_t)(p0 + i0) * BB)) + B * rr;
+    const BT* rv = reinterpret_cast<const BT*>(d + 2 * R::BLK + shift16(Lv + (size_t)(p0 + i0) * B)) + rr;
+    BT* out = Lv + (size_t)(p0 + i0) * B + r;
 #pragma unroll
     for (int t = 0; t < K; t++) {
-      const int i = i0 + t;
+      BT a[B];
+      load_row<BT, B>(a, lo + t * BB);
+      const BT ri = rv[t * B];
       BT s = 0;
 #pragma unroll
-      for (int q = 0; q < B; q++) s += mi[t][q] * __shfl_sync(0xffffffffu, v, q, LG);
-      if (i < n) {
-        v = xi[t] - s;
-        if (row) Lv[(size_t)(p0 + i) * B + r] = v;
+      for (int q = 0; q < B; q++) s += a[q] * __shfl_sync(0xffffffffu, v, q, LG);
+      if (i0 + t < n) {
+        v = ri - s;
+        if (row) out[t * B] = v;
       }
     }
-  };
-  {
-    BT ma[K][B], xa[K], mb[K][B], xb[K];
-    load_fwd(1, ma, xa);
-    for (int i0 = 1; i0 < nmax; i0 += 2 * K) {
-      if (i0 + K < nmax) load_fwd(i0 + K, mb, xb);
-      step_fwd(i0, ma, xa);
-      if (i0 + K >= nmax) break;
-      if (i0 + 2 * K < nmax) load_fwd(i0 + 2 * K, ma, xa);
-      step_fwd(i0 + K, mb, xb);
-    }
+    __syncwarp();
+    ask_fwd(c + S - 1);
   }
-  // backward: y_{n-1} = inv_{n-1} v_{n-1}, y_i = inv_i (v_i - up_{i+1} y_{i+1}); step j of the
-  // warp is position n-2-j of each line
+  // the copy engine reads v back: the stores above first
+  asm volatile("fence.proxy.async;" ::: "memory");
+  __syncwarp();
+  // backward: y_{n-1} = inv_{n-1} v_{n-1}, y_i = inv_i (v_i - up_{i+1} y_{i+1}); step j is position
+  // n - 2 - j of each line
+  auto ask_bwd = [&](int c) {
+    if (r != 0 || c >= chunks) return;
+    const int q = chunks + c, hi = n - 2 - c * K, lo = max(0, hi - K + 1), cnt = hi - lo + 1;
+    uint64_t* bar = &bars[q % S];
+    if (cnt <= 0) {
+      bar_expect(bar, 0);
+      return;
+    }
+    unsigned char* d = ring[q % S][g];
+    const BT *up = Lup + (size_t)(p0 + lo + 1) * BB, *iv = Linv + (size_t)(p0 + lo) * BB;
+    const BT* vv = Lv + (size_t)(p0 + lo) * B;
+    const unsigned lb = cnt * BB * sizeof(BT), vb = cnt * B * sizeof(BT);
+    bar_expect(bar, bulk_bytes(up, lb) + bulk_bytes(iv, lb) + bulk_bytes(vv, vb));
+    bulk_copy(d, up, lb, bar);
+    bulk_copy(d + R::BLK, iv, lb, bar);
+    bulk_copy(d + 2 * R::BLK, vv, vb, bar);
+  };
+  for (int c = 0; c < S - 1; c++) ask_bwd(c);
   BT yv = 0;
   {
     BT vq[B];
@@ -505,55 +583,39 @@ __global__ void __launch_bounds__(32 * LW) k_lsolve(Mesh m, Lines L, BT* __restr
       if (row) x[r * N + L.cv[p0 + n - 1]] = yv;
     }
   }
-  auto load_bwd = [&](int j0, BT(&ui)[K][B], BT(&ii)[K][B], BT(&vi)[K], int(&ci)[K]) {
+  for (int c = 0; c < chunks; c++) {
+    const int q0 = chunks + c, hi = n - 2 - c * K, l0 = max(0, hi - K + 1);
+    int cell[K];
+#pragma unroll
+    for (int t = 0; t < K; t++) cell[t] = hi - t >= 0 ? L.cv[p0 + hi - t] : 0;
+    ok = bar_wait(&bars[q0 % S], (q0 / S) & 1) && ok;
+    const unsigned char* d = ring[q0 % S][g];
+    const BT* up = reinterpret_cast<const BT*>(d + shift16(Lup + (size_t)(p0 + l0 + 1) * BB)) + B * rr;
+    const BT* iv = reinterpret_cast<const BT*>(d + R::BLK + shift16(Linv + (size_t)(p0 + l0) * BB)) + B * rr;
+    const BT* vv = reinterpret_cast<const BT*>(d + 2 * R::BLK + shift16(Lv + (size_t)(p0 + l0) * B)) + rr;
 #pragma unroll
     for (int t = 0; t < K; t++) {
-      const int i = n - 2 - (j0 + t);
-      if (i >= 0) {
-#pragma unroll
-        for (int q = 0; q < B; q++) {
-          ui[t][q] = Lup[(size_t)(p0 + i + 1) * BB + B * rr + q];
-          ii[t][q] = Linv[(size_t)(p0 + i) * BB + B * rr + q];
-        }
-        vi[t] = Lv[(size_t)(p0 + i) * B + rr];
-        ci[t] = L.cv[p0 + i];
-      } else {
-#pragma unroll
-        for (int q = 0; q < B; q++) ui[t][q] = ii[t][q] = BT(0);
-        vi[t] = BT(0);
-        ci[t] = 0;
-      }
-    }
-  };
-  auto step_bwd = [&](int j0, const BT(&ui)[K][B], const BT(&ii)[K][B], const BT(&vi)[K], const int(&ci)[K]) {
-#pragma unroll
-    for (int t = 0; t < K; t++) {
-      const int i = n - 2 - (j0 + t);
+      const int i = hi - t, k = max(i - l0, 0);  // past the line's front: any loaded record, unused
+      BT a[B], e[B];
+      load_row<BT, B>(a, up + k * BB);
+      load_row<BT, B>(e, iv + k * BB);
+      const BT vi = vv[k * B];
       BT s2 = 0;
 #pragma unroll
-      for (int q = 0; q < B; q++) s2 += ui[t][q] * __shfl_sync(0xffffffffu, yv, q, LG);
-      const BT a1 = vi[t] - s2;
+      for (int q = 0; q < B; q++) s2 += a[q] * __shfl_sync(0xffffffffu, yv, q, LG);
+      const BT a1 = vi - s2;
       BT s = 0;
 #pragma unroll
-      for (int q = 0; q < B; q++) s += ii[t][q] * __shfl_sync(0xffffffffu, a1, q, LG);
+      for (int q = 0; q < B; q++) s += e[q] * __shfl_sync(0xffffffffu, a1, q, LG);
       if (i >= 0) {
         yv = s;
-        if (row) x[r * N + ci[t]] = yv;
+        if (row) x[r * N + cell[t]] = yv;
       }
     }
-  };
-  {
-    BT ua[K][B], ia[K][B], va[K], ub[K][B], ib[K][B], vb[K];
-    int ca[K], cb[K];
-    load_bwd(0, ua, ia, va, ca);
-    for (int j0 = 0; j0 < nmax - 1; j0 += 2 * K) {
-      if (j0 + K < nmax - 1) load_bwd(j0 + K, ub, ib, vb, cb);
-      step_bwd(j0, ua, ia, va, ca);
-      if (j0 + K >= nmax - 1) break;
-      if (j0 + 2 * K < nmax - 1) load_bwd(j0 + 2 * K, ua, ia, va, ca);
-      step_bwd(j0 + K, ub, ib, vb, cb);
-    }
+    __syncwarp();
+    ask_bwd(c + S - 1);
   }
+  if (!ok && lane == 0) atomicOr(err, 8);
 }
 
 template <typename BT, int B>
@@ -566,9 +628,9 @@ void line_relax(const Mesh& m, State& st, const Lines& L, int sweeps, cudaStream
     // two columns at a time: most line cells have three or four couplings off their line.  The passes
     // and substitutions are plain launches: as programmatic dependents they measured 4-5% slower
     // (a pass's early blocks take the SMs of the substitutions, which are a chain of latencies)
-    k_sweep<BT, B, SWEEP_LINE, 2, sizeof(BT) == 4 ? 1600 / (B * SLICE) : 1>
-        <<<m.nslices, B * SLICE, 0, s>>>(m, st, xin, xout, it == 0, -1, nullptr, L.on_line, L.noff, L.off_end);
-    if (L.nlines) k_lsolve<BT, B><<<(L.nlines + LW * LPW - 1) / (LW * LPW), 32 * LW, 0, s>>>(m, L, xout);
+    k_sweep<BT, B, SWEEP_LINE, 2, sizeof(BT) == 4 ? 1600 / (B * SLICE) : 1><<<m.nslices, B * SLICE, 0, s>>>(
+        m, st, xin, xout, it == 0, -1, nullptr, L.line_pos, L.noff, L.off_end, (BT*)L.bv);
+    if (L.nlines) k_lsolve<BT, B><<<(L.nlines + LPW - 1) / LPW, 32, 0, s>>>(m, L, xout, st.err);
   }
 }
 

@@ -39,13 +39,14 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 enum { SWEEP_JACOBI = 0, SWEEP_GS = 1, SWEEP_LINE = 2 };
 
 // first: x is zero (the pass is Dinv b).  GS: slices (may be null: every slice) lists the slices
-// holding a cell of this colour.  LINE: on_line per cell, off the cell's number of
-// couplings off its line (its first columns), off_end per slice one past their last ELL row.
+// holding a cell of this colour.  LINE: line_pos the cell's position in the lines (-1:
+// on none), where its row goes into line_rhs; off the cell's number of couplings off its line (its
+// first columns), off_end per slice one past their last ELL row.
 template <typename BT, int B, int KIND, int COLS, int MINB>
 __global__ void __launch_bounds__(B * SLICE, MINB) k_sweep(Mesh m, State st, const BT* xin, BT* xout, int first, int color,
                                                      const int* __restrict__ slices,
-                                                     const uint8_t* __restrict__ on_line,
-                                                     const int* __restrict__ off, const int* __restrict__ off_end) {
+                                                     const int* __restrict__ line_pos, const int* __restrict__ off,
+                                                     const int* __restrict__ off_end, BT* line_rhs) {
   __shared__ BT xs[COLS][B][SLICE];
   __shared__ BT sacc[B][SLICE];
   pdl_trigger();
@@ -56,7 +57,8 @@ __global__ void __launch_bounds__(B * SLICE, MINB) k_sweep(Mesh m, State st, con
   bool active = c < N;
   if (KIND == SWEEP_GS) active = active && m.color[c] == color;
   if (KIND != SWEEP_LINE) active = active && st.case_active[m.case_of[c]];  // a frozen case does no work
-  const bool line = KIND == SWEEP_LINE && active && on_line[c];
+  const int lp = KIND == SWEEP_LINE && active ? line_pos[c] : -1;
+  const bool line = KIND == SWEEP_LINE && lp >= 0;
   BT acc = active ? (BT)st.b[(size_t)B * c + row] : (BT)0;
   constexpr bool PRE = COLS > 3;  // Dinv's row in registers before x is there
   BT di[B];
@@ -108,7 +110,8 @@ __global__ void __launch_bounds__(B * SLICE, MINB) k_sweep(Mesh m, State st, con
       for (int k = 0; k < B; k++) s += (PRE ? di[k] : ((const BT*)st.Dinv)[(size_t)(B * row + k) * N + c]) * sacc[k][lane];
       acc = s;
     }
-    xout[(size_t)row * N + c] = acc;
+    if (line) line_rhs[(size_t)B * lp + row] = acc;
+    else xout[(size_t)row * N + c] = acc;
   }
 }
 
@@ -158,7 +161,8 @@ void launch_sweep(const Mesh& m, const State& st, int grid, const BT* xin, BT* x
     kernel = grid <= fit_wide ? wide : grid <= fit_mid ? mid : narrow;
   }
   if (first) kernel = narrow;  // no matrix rows to request: Dinv b
-  launch_pass(kernel, grid, T, after_pass, s, m, st, xin, xout, (int)first, color, slices, nullptr, nullptr, nullptr);
+  launch_pass(kernel, grid, T, after_pass, s, m, st, xin, xout, (int)first, color, slices, nullptr, nullptr, nullptr,
+              nullptr);
 }
 
 // `sweeps` block Jacobi sweeps from zero: the result is in x0 (odd sweeps) or x1 (even)
