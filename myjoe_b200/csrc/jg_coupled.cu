@@ -684,13 +684,19 @@ struct VFC {
 };
 
 template <int NS>
-__device__ void visc_flux_c(double* Fv, VFC<NS>& vf, const VSideC<NS>& a, const VSideC<NS>& b, double mul,
+__device__ __forceinline__ void visc_flux_c(double* Fv, VFC<NS>& vf, const VSideC<NS>& a, const VSideC<NS>& b, double mul,
                             double mut, double lamOcp, double PrTurb, double kine_fa, const double* u_fa,
                             const double* diff, const double* diffTerm, double area, const double* nV, double smag,
                             const double* sV, double alpha) {
-  double g[3][3];
+  double g[3][3], ga[12], gb[12], ha[4], hb[4];
+  for (int i = 0; i < 12; i += 4) {
+    ld4(ga + i, a.gu + i);
+    ld4(gb + i, b.gu + i);
+  }
+  ld4(ha, a.gh);
+  ld4(hb, b.gh);
   for (int i = 0; i < 3; i++)
-    for (int j = 0; j < 3; j++) g[i][j] = 0.5 * (a.gu[3 * i + j] + b.gu[3 * i + j]);
+    for (int j = 0; j < 3; j++) g[i][j] = 0.5 * (ga[3 * i + j] + gb[3 * i + j]);
   double fC[3] = {nV[0] - alpha * sV[0], nV[1] - alpha * sV[1], nV[2] - alpha * sV[2]};
   const double aos = alpha / smag;  // the normal-derivative weight, one division for all terms
   double muT = mul + mut;
@@ -703,9 +709,9 @@ __device__ void visc_flux_c(double* Fv, VFC<NS>& vf, const VSideC<NS>& a, const 
   for (int i = 0; i < 3; i++) vf.tn[i] -= tmp * nV[i];
   for (int i = 0; i < 3; i++) Fv[1 + i] = -area * vf.tn[i];
   vf.keff = lamOcp + mut / PrTurb;
-  double enth = vf.keff * ((b.h - a.h) * aos + 0.5 * ((a.gh[0] + b.gh[0]) * fC[0] +
-                                                             (a.gh[1] + b.gh[1]) * fC[1] +
-                                                             (a.gh[2] + b.gh[2]) * fC[2]));
+  double enth = vf.keff * ((b.h - a.h) * aos + 0.5 * ((ha[0] + hb[0]) * fC[0] +
+                                                             (ha[1] + hb[1]) * fC[1] +
+                                                             (ha[2] + hb[2]) * fC[2]));
   double psi = muT * ((b.k - a.k) * aos);
   Fv[4] = -area * (enth + vf.tn[0] * u_fa[0] + vf.tn[1] * u_fa[1] + vf.tn[2] * u_fa[2] + psi);
   for (int s = 0; s < NS; s++) {
@@ -764,11 +770,14 @@ template <int NS>
 __device__ __forceinline__ CState<NS> cell_c(const Mesh& m, const Params& p, const State& st, const Turb& t, int c,
                                              bool sst) {
   CState<NS> s;
-  s.rho = st.q[5 * c];
-  for (int i = 0; i < 3; i++) s.u[i] = st.prim[8 * c + i];
-  s.p = st.prim[8 * c + 3];
-  s.T = st.prim[8 * c + 4];
-  s.h = st.prim[8 * c + 5];
+  double a[4], b[4];
+  ld4(a, &st.prim[(size_t)8 * c]);
+  ld4(b, &st.prim[(size_t)8 * c + 4]);
+  for (int i = 0; i < 3; i++) s.u[i] = a[i];
+  s.p = a[3];
+  s.T = b[0];
+  s.h = b[1];
+  s.rho = b[3];
   s.gam = p.gamma;
   for (int q = 0; q < NS; q++) s.sc[q] = t.phi[(size_t)q * m.ncv + c];
   s.k = sst ? s.sc[0] : 0.0;
@@ -795,15 +804,16 @@ __device__ __forceinline__ CState<NS> recon_c(const Mesh& m, const Params& p, co
                                               int f, bool sst) {
   CState<NS> s = cell_c<NS>(m, p, st, t, c, sst);
   if (!p.second_order) return s;
-  double r0[3];
-  for (int i = 0; i < 3; i++) r0[i] = m.x_fa[3 * f + i] - m.x_cv[3 * c + i];
-  double rr = s.rho + dot3(r0, &st.grho[GS * c]);
-  double pp = s.p + dot3(r0, &st.gp[GS * c]);
+  double r0[3], g[GS];
+  for (int i = 0; i < GS; i += 4) ld4(g + i, &st.gu[(size_t)GS * c + i]);
+  cell_to_face(m, c, f, r0);
+  double rr = s.rho + dot3(r0, g + 9);
+  double pp = s.p + dot3(r0, g + 12);
   if ((pp <= 0.0) || (rr <= 0.0)) {
     pp = s.p;
     rr = s.rho;
   } else {
-    for (int i = 0; i < 3; i++) s.u[i] += dot3(r0, &st.gu[GS * c + 3 * i]);
+    for (int i = 0; i < 3; i++) s.u[i] += dot3(r0, &g[3 * i]);
     for (int q = 0; q < NS; q++) s.sc[q] += dot3(r0, &t.grad_phi[((size_t)q * m.ncv + c) * 3]);
   }
   s.rho = rr;
@@ -817,10 +827,13 @@ template <int NS>
 __device__ __forceinline__ VSideC<NS> vcell_c(const Mesh& m, const State& st, const Turb& t, const Params& p, int c,
                                               bool sst) {
   VSideC<NS> v;
-  v.rho = st.q[5 * c];
-  for (int i = 0; i < 3; i++) v.u[i] = st.prim[8 * c + i];
-  v.h = st.prim[8 * c + 5];
-  v.T = st.prim[8 * c + 4];
+  double a[4], b[4];
+  ld4(a, &st.prim[(size_t)8 * c]);
+  ld4(b, &st.prim[(size_t)8 * c + 4]);
+  for (int i = 0; i < 3; i++) v.u[i] = a[i];
+  v.T = b[0];
+  v.h = b[1];
+  v.rho = b[3];
   v.gam = p.gamma;
   for (int q = 0; q < NS; q++) {
     v.sc[q] = t.phi[(size_t)q * m.ncv + c];
@@ -892,12 +905,67 @@ __device__ void block_inverse_n(double* A, double* Ai) {
   }
 }
 
+// model sources: sourceHookRansTurbCoupled (TurbModel_SA.h:359-434; TurbModel_KOMSST.h:306-340), into
+// the scalars' rows of the residual, and the derivatives the diagonal block takes
+template <int MODEL>
+__device__ __forceinline__ void model_source(const Mesh& m, const State& st, const Turb& t, int c, double* rhs,
+                                             double* dsrc) {
+  constexpr bool SST = MODEL == JG_TURB_SST;
+  const int N = m.ncv;
+  const double rho = st.q[5 * c], vol = m.vol[c];
+  if constexpr (!SST) {
+    double mue = face_avg_c(m, st.mul_fa, c);
+    double Om = fmax(t.vortMag[c], 1.e-8);
+    double Strainrate = fmax(t.strMag[c], 1.e-8);
+    double d = t.wd[c];
+    double nu = t.phi[c];
+    double chi = nu * rho / mue;
+    double chi_3 = pow(chi, 3.0);
+    double inv_K2d2 = 1.0 / (SA_K2 * d * d);
+    double fv1 = chi_3 / (chi_3 + SA_CV1_3);
+    double fv2 = 1.0 - chi / (1.0 + chi * fv1);
+    double S = fmax(Om + fmin(0.0, Strainrate - Om) * 0.0, 0.0);
+    double Shat = S + nu * fv2 * inv_K2d2;
+    double inv_Shat = 1.0 / fmax(Shat, 1.0e-8);
+    double r = fmin(nu * inv_Shat * inv_K2d2, 10.0);
+    double g = r + SA_CW2 * (pow(r, 6.0) - r);
+    double g_6 = pow(g, 6.0);
+    double fw = g * pow((1.0 + SA_CW3_6) / (g_6 + SA_CW3_6), 1.0 / 6.0);
+    double H1 = SA_CB1 * Shat * nu;
+    double H2 = -SA_CW1 * fw * nu * nu / sq(d);
+    double H3 = SA_CB2 / SA_SIGMA * dot3(&t.grad_phi[3 * c], &t.grad_phi[3 * c]);
+    rhs[5] += rho * vol * (H1 + H2 + H3);
+    double d_H2 = -2.0 * SA_CW1 * fw * nu / sq(d);
+    dsrc[0] = (0.0 + d_H2) * vol;
+  } else {
+    double k = t.phi[c], om = t.phi[N + c];
+    double F1 = t.F1[c];
+    double alfa_1 = SST_B1 / SST_BS - SST_SO1 * sq(0.41) / sqrt(SST_BS);
+    double alfa_2 = SST_B2 / SST_BS - SST_SO2 * sq(0.41) / sqrt(SST_BS);
+    double alfa = F1 * alfa_1 + (1.0 - F1) * alfa_2;
+    double beta = F1 * SST_B1 + (1.0 - F1) * SST_B2;
+    double zeta = fmin(1.0 / om, SST_A1 / (t.vortMag[c] * t.F2[c]));
+    double mut = fmin(fmax(rho * k * zeta, 1.0e-8), 1.0e5);
+    double str = t.strMag[c], div = t.diverg[c];
+    double Pk = fmax(mut * str * str - 2. / 3. * rho * k * div, 0.0);
+    Pk = fmin(Pk, 20.0 * SST_BS * rho * k * om);
+    rhs[5] += (Pk - SST_BS * rho * om * k) * vol;
+    zeta = fmax(om, t.vortMag[c] * t.F2[c] / SST_A1);
+    Pk = fmax(str * str - 2. / 3. * zeta * div, 0.0);
+    rhs[6] += (alfa * rho * Pk + (1.0 - F1) * t.crossDiff[c] - beta * rho * om * om) * vol;
+    dsrc[0] = -SST_BS * om * vol;
+    dsrc[1] = -2.0 * beta * om * vol;
+  }
+}
+
 // ---------------------------------------------------------------------------
 // face loop: calcRhsCoupled (fluxes, boundary zones, model sources) + the
 // implicit-step epilogue (vol/dt, under-relaxed rhs, D^-1)
 // ---------------------------------------------------------------------------
-template <typename BT, int MODEL, int FK>
-__global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb t, int implicit, int for_step) {
+// IMPL: with the Jacobian blocks (the AUSM family); else the residual alone
+template <typename BT, int MODEL, int FK, bool IMPL>
+__global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb t, int for_step) {
+  constexpr bool implicit = IMPL;
   constexpr int NS = TM<MODEL>::NS, B = TM<MODEL>::B, BB = TM<MODEL>::BB;
   constexpr bool SST = MODEL == JG_TURB_SST;
   extern __shared__ double sD[];  // [BB][blockDim.x]
@@ -908,7 +976,8 @@ __global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb
   const bool only_p = p.symm_bc == JG_SYMM_ANALYTICAL;
   double rhs[B];
   for (int i = 0; i < B; i++) rhs[i] = 0.0;
-  for (int e = 0; e < BB; e++) sD[e * bd + tid] = 0.0;
+  if (implicit)
+    for (int e = 0; e < BB; e++) sD[e * bd + tid] = 0.0;
   BT* O = (BT*)st.O;
   double F[B];
   double one[NS], dfa[NS], dterm[NS];
@@ -1094,55 +1163,11 @@ __global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb
     }
   }
   gravity_rhs(p, m, st, c, rhs);  // sourceHookCoupled
-  // model sources: sourceHookRansTurbCoupled (TurbModel_SA.h:359-434; TurbModel_KOMSST.h:306-340)
   double dsrc[NS];
-  {
-    const double rho = st.q[5 * c], vol = m.vol[c];
-    if constexpr (!SST) {
-      double mue = face_avg_c(m, st.mul_fa, c);
-      double Om = fmax(t.vortMag[c], 1.e-8);
-      double Strainrate = fmax(t.strMag[c], 1.e-8);
-      double d = t.wd[c];
-      double nu = t.phi[c];
-      double chi = nu * rho / mue;
-      double chi_3 = pow(chi, 3.0);
-      double inv_K2d2 = 1.0 / (SA_K2 * d * d);
-      double fv1 = chi_3 / (chi_3 + SA_CV1_3);
-      double fv2 = 1.0 - chi / (1.0 + chi * fv1);
-      double S = fmax(Om + fmin(0.0, Strainrate - Om) * 0.0, 0.0);
-      double Shat = S + nu * fv2 * inv_K2d2;
-      double inv_Shat = 1.0 / fmax(Shat, 1.0e-8);
-      double r = fmin(nu * inv_Shat * inv_K2d2, 10.0);
-      double g = r + SA_CW2 * (pow(r, 6.0) - r);
-      double g_6 = pow(g, 6.0);
-      double fw = g * pow((1.0 + SA_CW3_6) / (g_6 + SA_CW3_6), 1.0 / 6.0);
-      double H1 = SA_CB1 * Shat * nu;
-      double H2 = -SA_CW1 * fw * nu * nu / sq(d);
-      double H3 = SA_CB2 / SA_SIGMA * dot3(&t.grad_phi[3 * c], &t.grad_phi[3 * c]);
-      rhs[5] += rho * vol * (H1 + H2 + H3);
-      double d_H2 = -2.0 * SA_CW1 * fw * nu / sq(d);
-      dsrc[0] = (0.0 + d_H2) * vol;
-    } else {
-      double k = t.phi[c], om = t.phi[N + c];
-      double F1 = t.F1[c];
-      double alfa_1 = SST_B1 / SST_BS - SST_SO1 * sq(0.41) / sqrt(SST_BS);
-      double alfa_2 = SST_B2 / SST_BS - SST_SO2 * sq(0.41) / sqrt(SST_BS);
-      double alfa = F1 * alfa_1 + (1.0 - F1) * alfa_2;
-      double beta = F1 * SST_B1 + (1.0 - F1) * SST_B2;
-      double zeta = fmin(1.0 / om, SST_A1 / (t.vortMag[c] * t.F2[c]));
-      double mut = fmin(fmax(rho * k * zeta, 1.0e-8), 1.0e5);
-      double str = t.strMag[c], div = t.diverg[c];
-      double Pk = fmax(mut * str * str - 2. / 3. * rho * k * div, 0.0);
-      Pk = fmin(Pk, 20.0 * SST_BS * rho * k * om);
-      rhs[5] += (Pk - SST_BS * rho * om * k) * vol;
-      zeta = fmax(om, t.vortMag[c] * t.F2[c] / SST_A1);
-      Pk = fmax(str * str - 2. / 3. * zeta * div, 0.0);
-      rhs[6] += (alfa * rho * Pk + (1.0 - F1) * t.crossDiff[c] - beta * rho * om * om) * vol;
-      dsrc[0] = -SST_BS * om * vol;
-      dsrc[1] = -2.0 * beta * om * vol;
-    }
-  }
+  model_source<MODEL>(m, st, t, c, rhs, dsrc);
   for (int i = 0; i < B; i++) st.rhs[(size_t)B * c + i] = rhs[i];
+  if (for_step)
+    for (int i = 0; i < B; i++) st.b[(size_t)B * c + i] = p.under_relax * rhs[i];
   if (implicit) {
     double Dm[BB];
     for (int e = 0; e < BB; e++) Dm[e] = sD[e * bd + tid];
@@ -1151,7 +1176,6 @@ __global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb
     if (for_step) {
       double tmp = m.vol[c] / st.local_dt[c];
       for (int i = 0; i < B; i++) Dm[(B + 1) * i] += tmp;
-      for (int i = 0; i < B; i++) st.b[(size_t)B * c + i] = p.under_relax * rhs[i];
     }
     BT* Dg = (BT*)st.D;
     for (int e = 0; e < BB; e++) Dg[(size_t)e * m.ncv + c] = (BT)Dm[e];
@@ -1162,6 +1186,394 @@ __global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb
       for (int e = 0; e < BB; e++) Dig[(size_t)e * m.ncv + c] = (BT)Di[e];
     }
   }
+}
+
+// ---------------------------------------------------------------------------
+// The Jacobian blocks with HLLC, row by row: every row of a face's two matrices goes into the cell's
+// diagonal block (shared memory) and its off-diagonal block as soon as it is formed, so no thread
+// holds a B x B matrix.  Formed whole beside the residual, the matrices cost 255 registers, spills
+// and two blocks per SM (100k cells 6x6 FP64: 429 us for both -> 71 residual + 197 here + 24 inverse; 7x7
+// FP32 393 -> 88 + 133 + 24 at 70k; capped at 168 registers the rows spill: 250 and 220).  Each entry is the expression of
+// matrices_hllc_c; of the scalars' columns only the diagonal entries differ from zero (dp/dscal = 0),
+// so the dU/dQ products with the others are left out.
+// ---------------------------------------------------------------------------
+// emit(r, aL, aR): rows r of A_L and A_R
+template <int NS, typename Emit>
+__device__ __forceinline__ void hllc_rows_c(const CState<NS>& L, const CState<NS>& R, double area, const double* nV,
+                                            Emit&& emit) {
+  constexpr int B = 5 + NS;
+  const double unL = dot3(L.u, nV), uLuL = dot3(L.u, L.u), cL = sqrt(L.gam * L.p / L.rho);
+  const double hL = L.h + L.k, rhoeL = (hL + 0.5 * uLuL) * L.rho - L.p;
+  const double unR = dot3(R.u, nV), uRuR = dot3(R.u, R.u), cR = sqrt(R.gam * R.p / R.rho);
+  const double hR = R.h + R.k, rhoeR = (hR + 0.5 * uRuR) * R.rho - R.p;
+  const double Rrho = sqrt(R.rho / L.rho);
+  const double tmp = 1.0 / (1.0 + Rrho);
+  double vR[3];
+  for (int i = 0; i < 3; i++) vR[i] = tmp * (L.u[i] + R.u[i] * Rrho);
+  const double uRoe = dot3(vR, nV);
+  const double gpr = tmp * ((L.gam * L.p / L.rho + 0.5 * (L.gam - 1.0) * uLuL) +
+                            (R.gam * R.p / R.rho + 0.5 * (R.gam - 1.0) * uRuR) * Rrho);
+  const double cRoe = sqrt(gpr - ((L.gam + R.gam) * 0.5 - 1.0) * 0.5 * dot3(vR, vR));
+  const double sL = fmin(uRoe - cRoe, unL - cL);
+  const double sR = fmax(uRoe + cRoe, unR + cR);
+  const double invrhotld = 1.0 / (R.rho * (sR - unR) - L.rho * (sL - unL));
+  const double sM = (L.p - R.p - L.rho * unL * (sL - unL) + R.rho * unR * (sR - unR)) /
+                    (R.rho * (sR - unR) - L.rho * (sL - unL));
+  const double pS = R.rho * (unR - sR) * (unR - sM) + R.p;
+  const double nA[3] = {nV[0] * area, nV[1] * area, nV[2] * area};
+  // the upwind side: the star state's, or the whole flux's when it is supersonic
+  const bool left = sM >= 0.0;
+  const bool sonic = left ? sL > 0.0 : !(sR >= 0.0);
+  const double u[3] = {left ? L.u[0] : R.u[0], left ? L.u[1] : R.u[1], left ? L.u[2] : R.u[2]};
+  const double pp = left ? L.p : R.p, rho = left ? L.rho : R.rho, hh = left ? hL : hR, gamma = left ? L.gam : R.gam;
+  const double un = left ? unL : unR, rhoe = left ? rhoeL : rhoeR, sS = left ? sL : sR;
+  double sc[NS];
+  for (int s = 0; s < NS; s++) sc[s] = left ? L.sc[s] : R.sc[s];
+  // calcJacobianCoupled_HLLC's constants
+  const double kapm1 = gamma - 1.0;
+  const double nVel[3] = {u[0] * nA[0], u[1] * nA[1], u[2] * nA[2]};
+  const double U_k = nVel[0] + nVel[1] + nVel[2];
+  const double vSquHlf = 0.5 * dot3(u, u);
+  // of the upwind side (S) and the other (O): area OmSMp1 dSM/dU and the mass factor of the star state
+  double dS[5], dO[5], mS = 0.0, mO = 0.0, rhoS = 0.0, rhouS[3], e4 = 0.0, OmSM = -1.0, diag = 0.0;
+  if (!sonic) {
+    const double Om = 1.0 / (sS - sM), d = sS - un;
+    rhoS = rho * d * Om;
+    for (int i = 0; i < 3; i++) rhouS[i] = (rho * u[i] * d + (pS - pp) * nV[i]) * Om;
+    const double rhoeS = (d * rhoe - pp * un + pS * sM) * Om;
+    double dl[B], dr[B];
+    dsmdu_c<NS>(dl, L.u, L.p, L.rho, hL, nV, L.gam, sM, sL, invrhotld, 1.0);
+    dsmdu_c<NS>(dr, R.u, R.p, R.rho, hR, nV, R.gam, sM, sR, invrhotld, -1.0);
+    OmSM = Om * sM;
+    const double OmSMp1 = OmSM + 1.0, mL = R.rho * (sR - unR), mR = L.rho * (sL - unL);
+    for (int i = 0; i < 5; i++) {
+      dS[i] = area * OmSMp1 * (left ? dl[i] : dr[i]);
+      dO[i] = area * OmSMp1 * (left ? dr[i] : dl[i]);
+    }
+    mS = left ? mL : mR;
+    mO = left ? mR : mL;
+    e4 = rhoeS + pS;
+    diag = area * Om * sM * sS;
+  }
+#pragma unroll
+  for (int r = 0; r < B; r++) {
+    // row r of the upwind side's flux Jacobian
+    double J[5], js = 0.0;
+    if (r == 0) {
+      J[0] = 0.0; J[1] = nA[0]; J[2] = nA[1]; J[3] = nA[2]; J[4] = 0.0;
+    } else if (r < 4) {
+      const int q = r - 1;
+      J[0] = -u[q] * U_k + nA[q] * (kapm1 * vSquHlf + gamma * pp / rho - kapm1 * hh);
+#pragma unroll
+      for (int i = 0; i < 3; i++) J[1 + i] = (q == i) ? (2.0 - gamma) * nVel[q] + U_k : u[q] * nA[i] - kapm1 * u[i] * nA[q];
+      J[4] = kapm1 * nA[q];
+    } else if (r == 4) {
+      J[0] = U_k * ((gamma - 2.0) * vSquHlf - gamma * (hh - pp / rho));
+#pragma unroll
+      for (int i = 0; i < 3; i++) J[1 + i] = (hh + vSquHlf) * nA[i] - kapm1 * u[i] * U_k;
+      J[4] = gamma * U_k;
+    } else {
+      J[0] = 0.0;
+#pragma unroll
+      for (int i = 0; i < 3; i++) J[1 + i] = sc[r >= 5 ? r - 5 : 0] * nA[i];
+      J[4] = 0.0;
+      js = rho * U_k;
+    }
+    double own[B], oth[B];  // the upwind side's and the other side's row
+#pragma unroll
+    for (int i = 0; i < B; i++) own[i] = oth[i] = 0.0;
+    if (sonic) {
+#pragma unroll
+      for (int i = 0; i < 5; i++) own[i] = J[i];
+      if (r >= 5) own[r] = js;
+    } else {
+      // calcSubSonicJacobianCoupled_HLLC's star-state factor of the row
+      double rrS, rrO;
+      if (r == 0) {
+        rrS = rrO = rhoS;
+      } else if (r < 4) {
+        rrS = rhouS[r >= 1 && r < 4 ? r - 1 : 0] + mS * nV[r >= 1 && r < 4 ? r - 1 : 0];
+        rrO = rhouS[r >= 1 && r < 4 ? r - 1 : 0] + mO * nV[r >= 1 && r < 4 ? r - 1 : 0];
+      } else if (r == 4) {
+        rrS = e4 + mS * sM;
+        rrO = e4 + mO * sM;
+      } else {
+        rrS = rrO = rhoS * sc[r >= 5 ? r - 5 : 0];
+      }
+#pragma unroll
+      for (int i = 0; i < 5; i++) {
+        own[i] = -OmSM * J[i] + dS[i] * rrS;
+        oth[i] = dO[i] * rrO;
+      }
+      if (r < 5) {
+        own[r] += diag;
+      } else {
+        own[0] += diag * sc[r >= 5 ? r - 5 : 0];
+        own[r] = -OmSM * js + diag * rho;
+      }
+    }
+    if (r >= 5) {  // dU/dQ of the scalar's column
+      own[0] -= sc[r >= 5 ? r - 5 : 0] / rho * own[r];
+      own[r] /= rho;
+    }
+    if (left) emit(r, own, oth);
+    else emit(r, oth, own);
+  }
+}
+
+// the viscous matrix of one side (visc_jac_c_add) reduced to what each row adds: rows 1-3 get a in
+// column 0 and b on the diagonal, row 4 gets w, a scalar's row s0 in column 0 and s1 on the diagonal
+template <int NS>
+struct VJacC {
+  double a[3], b, w[5], s0[NS], s1[NS];
+};
+template <int NS>
+__device__ __forceinline__ VJacC<NS> vjac_c(int side, const VFC<NS>& vf, const VSideC<NS>& v, const double* u_fa,
+                                            double R, double area) {
+  VJacC<NS> o;
+  const double sg = side ? -1.0 : 1.0;
+  const double d11 = sg * vf.muT * vf.aas;
+  const double d41 = -area * vf.tn[0] * 0.5 + u_fa[0] * d11;
+  const double d42 = -area * vf.tn[1] * 0.5 + u_fa[1] * d11;
+  const double d43 = -area * vf.tn[2] * 0.5 + u_fa[2] * d11;
+  const double d44 = sg * vf.keff * vf.aas;
+  const double iR = 1.0 / v.rho;
+  const double q10 = -iR * v.u[0], q20 = -iR * v.u[1], q30 = -iR * v.u[2];
+  const double q40 = iR * v.gam * (-v.h - v.k + R * v.T + 0.5 * dot3(v.u, v.u));
+  const double q41 = -iR * v.u[0] * v.gam, q42 = -iR * v.u[1] * v.gam, q43 = -iR * v.u[2] * v.gam, q44 = iR * v.gam;
+  o.a[0] = d11 * q10;
+  o.a[1] = d11 * q20;
+  o.a[2] = d11 * q30;
+  o.b = d11 * iR;
+  o.w[0] = d41 * q10 + d42 * q20 + d43 * q30 + d44 * q40;
+  o.w[1] = d41 * iR + d44 * q41;
+  o.w[2] = d42 * iR + d44 * q42;
+  o.w[3] = d43 * iR + d44 * q43;
+  o.w[4] = d44 * q44;
+  for (int s = 0; s < NS; s++) {
+    const double dss = sg * vf.dd[s] * vf.aas;
+    o.s0[s] = dss * (-iR * v.sc[s]);
+    o.s1[s] = dss * iR;
+  }
+  return o;
+}
+template <int NS, typename Acc>
+__device__ __forceinline__ void vjac_c_row(Acc acc, int r, double sgn, const VJacC<NS>& v) {
+  if (r >= 1 && r <= 3) {
+    acc[0] += sgn * v.a[r - 1];
+    acc[r] += sgn * v.b;
+  } else if (r == 4) {
+    for (int k = 0; k < 5; k++) acc[k] += sgn * v.w[k];
+  } else if (r >= 5) {
+    acc[0] += sgn * v.s0[r >= 5 ? r - 5 : 0];
+    acc[r] += sgn * v.s1[r >= 5 ? r - 5 : 0];
+  }
+}
+
+constexpr int TBJ = 64;  // cells per block of k_jac_c
+template <typename BT, int MODEL>
+__global__ void __launch_bounds__(TBJ, 4) k_jac_c(Mesh m, Params p, State st, Turb t, int for_step, double* dfull) {
+  constexpr int NS = TM<MODEL>::NS, B = TM<MODEL>::B, BB = TM<MODEL>::BB;
+  constexpr bool SST = MODEL == JG_TURB_SST;
+  __shared__ double sD[BB][TBJ];
+  const int tid = threadIdx.x, c = blockIdx.x * TBJ + tid;
+  if (c >= m.ncv || !st.case_active[m.case_of[c]]) return;  // a frozen case keeps its arrays
+  const int nf = m.nfa;
+  const bool only_p = p.symm_bc == JG_SYMM_ANALYTICAL;
+  for (int e = 0; e < BB; e++) sD[e][tid] = 0.0;
+  BT* O = (BT*)st.O;
+  const int slice = c / SLICE, lane = c % SLICE;
+  double F[B], one[NS], dfa[NS], dterm[NS];
+  for (int q = 0; q < NS; q++) one[q] = 1.0;
+  for (int k = m.slot_i[c]; k < m.slot_i[c + 1]; k++) {
+    const Slot s = m.slots[k];
+    const int f = s.f;
+    double nV[3], area;
+    unit_normal(m, f, nV, area);
+    for (int q = 0; q < NS; q++) dfa[q] = t.diff[(size_t)q * nf + f];
+    VFC<NS> vf;
+    if (s.nb >= 0) {
+      const int c0 = s.side == 0 ? c : s.nb;
+      const int c1 = s.side == 0 ? s.nb : c;
+      const bool first = s.side == 0;
+      VJacC<NS> vd, vo;
+      {
+        VSideC<NS> v0 = vcell_c<NS>(m, st, t, p, c0, SST), v1 = vcell_c<NS>(m, st, t, p, c1, SST);
+        double sV[3], smag;
+        cell_to_cell(m, f, sV, smag);
+        const double alpha = dot3(nV, sV);
+        double ufa[3] = {0.5 * (v0.u[0] + v1.u[0]), 0.5 * (v0.u[1] + v1.u[1]), 0.5 * (v0.u[2] + v1.u[2])};
+        double kine_fa = 0.0;
+        if (SST) {
+          double d0[3], d1[3];
+          cell_to_face(m, c0, f, d0);
+          cell_to_face(m, c1, f, d1);
+          const double w0 = sqrt(dot3(d0, d0)), w1 = sqrt(dot3(d1, d1));
+          kine_fa = (w1 * v0.k + w0 * v1.k) / (w0 + w1);
+        }
+        visc_flux_c<NS>(F, vf, v0, v1, st.mul_fa[f], st.mut_fa[f], st.lam_fa[f], p.PrTurb, kine_fa, ufa, dfa, one,
+                        area, nV, smag, sV, alpha);
+        // row of c0: D += A0, O += A1 ; row of c1: D -= A1, O -= A0  (JoeWithModels.cpp:5110-5127)
+        vd = first ? vjac_c<NS>(0, vf, v0, ufa, p.R, area) : vjac_c<NS>(1, vf, v1, ufa, p.R, area);
+        vo = first ? vjac_c<NS>(1, vf, v1, ufa, p.R, area) : vjac_c<NS>(0, vf, v0, ufa, p.R, area);
+      }
+      const CState<NS> L0 = cell_c<NS>(m, p, st, t, c0, SST), R0 = cell_c<NS>(m, p, st, t, c1, SST);
+      BT* ob = O + (size_t)(m.ell_off[slice] + s.col) * BB * SLICE + lane;
+      const double vsg = first ? 1.0 : -1.0;
+      // row of c0: D += Apl, O = Ami ; row of c1: D -= Ami, O = -Apl
+      hllc_rows_c<NS>(L0, R0, area, nV, [&](int r, const double* aL, const double* aR) {
+        double orow[B], drow[B];
+#pragma unroll
+        for (int j = 0; j < B; j++) {
+          drow[j] = 0.0;
+          orow[j] = first ? aR[j] : -aL[j];
+        }
+        vjac_c_row<NS>(drow, r, vsg, vd);
+        vjac_c_row<NS>(orow, r, vsg, vo);
+#pragma unroll
+        for (int j = 0; j < B; j++) {
+          sD[B * r + j][tid] = (sD[B * r + j][tid] + (first ? aL[j] : -aR[j])) + drow[j];
+          ob[(B * r + j) * SLICE] = (BT)orow[j];
+        }
+      });
+    } else {
+      // boundary face; the cell is cvofa[f][0] (JoeWithModels.cpp:5139-5799)
+      const DevZone z = m.zones[m.bzone[f]];
+      for (int q = 0; q < NS; q++) dterm[q] = (z.scal_bc & ((1 << q) | (1 << (4 + q)))) ? 1.0 : 0.0;
+      CState<NS> Bs = bfa_c<NS>(m, p, st, t, f);
+      const bool sym = z.kind == JG_BC_SYMMETRY, neu = z.kind == JG_BC_NEUMANN, wall = z.kind == JG_BC_WALL;
+      if (SST && !wall) Bs.k = Bs.sc[0];  // the wall keeps the face kinetic energy at 0
+      auto add = [&](int r, const double* aL, const double* aR, bool both) {
+#pragma unroll
+        for (int j = 0; j < B; j++) sD[B * r + j][tid] += both ? aL[j] + aR[j] : aL[j];
+      };
+      if ((sym || wall) && p.symm_bc != JG_SYMM_NEW_NUMERIC && only_p) {
+        // the pressure flux alone: its derivatives in the momentum rows
+        const double uLuL = dot3(Bs.u, Bs.u), hL = Bs.h + Bs.k, g = Bs.gam;
+        const double dpdrho = 0.5 * (g - 1.0) * uLuL - (g - 1.0) * hL + g * Bs.p / Bs.rho;
+        for (int r = 0; r < 3; r++) {
+          sD[B * (1 + r)][tid] += dpdrho * nV[r] * area;
+          for (int i = 0; i < 3; i++) sD[B * (1 + r) + 1 + i][tid] += -(g - 1.0) * Bs.u[i] * nV[r] * area;
+          sD[B * (1 + r) + 4][tid] += (g - 1.0) * nV[r] * area;
+        }
+      } else {
+        // SYMMETRY, WALL and NEUMANN at the boundary state (SYMM_BC NEW_NUMERIC adds the outer side's), the
+        // others at the cell state against it
+        const bool bstate = sym || wall || neu, both = bstate && p.symm_bc == JG_SYMM_NEW_NUMERIC;
+        const CState<NS> L0 = bstate ? Bs : cell_c<NS>(m, p, st, t, c, SST);
+        hllc_rows_c<NS>(L0, Bs, area, nV, [&](int r, const double* aL, const double* aR) { add(r, aL, aR, both); });
+      }
+      if (sym) continue;
+      VSideC<NS> v0 = vcell_c<NS>(m, st, t, p, c, SST), vb = vbfa_c<NS>(st, p, f, c);
+      double sV[3], smag, alpha = 1.0;
+      cell_to_face(m, c, f, sV);
+      if (neu || wall) {
+        smag = fabs(dot3(sV, nV));
+        for (int i = 0; i < 3; i++) sV[i] = nV[i];
+      } else {
+        smag = sqrt(dot3(sV, sV));
+        for (int i = 0; i < 3; i++) sV[i] /= smag;
+        alpha = dot3(nV, sV);
+      }
+      if (neu) {
+        for (int q = 0; q < NS; q++) vb.sc[q] = Bs.sc[q];
+        vb.k = Bs.k;
+        v0 = vb;
+      } else if (!wall) {
+        vb.k = Bs.k;
+      }
+      const double* dt = neu ? one : dterm;
+      visc_flux_c<NS>(F, vf, v0, vb, st.mul_fa[f], wall ? 0.0 : st.mut_fa[f], st.lam_fa[f], p.PrTurb,
+                      wall ? 0.0 : Bs.k, vb.u, dfa, dt, area, nV, smag, sV, alpha);
+      const VJacC<NS> vd = vjac_c<NS>(0, vf, v0, vb.u, p.R, area);
+#pragma unroll
+      for (int r = 1; r < B; r++) {
+        double drow[B];
+        for (int j = 0; j < B; j++) drow[j] = 0.0;
+        vjac_c_row<NS>(drow, r, 1.0, vd);
+        for (int j = 0; j < B; j++) sD[B * r + j][tid] += drow[j];
+      }
+    }
+  }
+  double rhs[B], dsrc[NS];
+  for (int i = 0; i < B; i++) rhs[i] = 0.0;
+  model_source<MODEL>(m, st, t, c, rhs, dsrc);
+  // the diagonal block: gravity, the sources' derivatives and vol / dt, left in shared memory
+  if (p.has_gravity) {
+    const double vol = m.vol[c];
+    for (int i = 0; i < 3; i++) {
+      sD[B * (1 + i)][tid] -= vol * p.gravity[i];
+      sD[B * 4 + 1 + i][tid] -= vol * p.gravity[i];
+    }
+  }
+  for (int q = 0; q < NS; q++) sD[(B + 1) * (5 + q)][tid] -= dsrc[q];
+  if (for_step) {
+    const double tmp = m.vol[c] / st.local_dt[c];
+    for (int i = 0; i < B; i++) sD[(B + 1) * i][tid] += tmp;
+  }
+  double* dd = dfull + c;
+  BT* Dg = (BT*)st.D;
+  for (int e = 0; e < BB; e++) {
+    Dg[(size_t)e * m.ncv + c] = (BT)sD[e][tid];
+    if (for_step && sizeof(BT) == 4) dd[(size_t)e * m.ncv] = sD[e][tid];
+  }
+}
+
+// Dinv of the diagonal blocks, ludeco / luinv (UgpWithCv.cpp:2489-2577) with B threads per cell: thread r
+// takes the block's rows and columns r, 32 cells a block, the block in shared memory.  In the thread
+// that formed the block the two B x B arrays went through local memory entry by entry.
+template <typename BT, int B>
+__global__ void __launch_bounds__(32 * B) k_inv_c(Mesh m, State st, const double* __restrict__ D) {
+  constexpr int BB = B * B;
+  __shared__ double A[BB][32];
+  const int lane = threadIdx.x % 32, r = threadIdx.x / 32, N = m.ncv;
+  const int c = blockIdx.x * 32 + lane;
+  const bool on = c < N && st.case_active[m.case_of[c]];
+  if (on)
+#pragma unroll
+    for (int k = 0; k < B; k++) A[B * r + k][lane] = D[(size_t)(B * r + k) * N + c];
+  __syncthreads();
+  if (on && r > 0) A[r][lane] /= A[0][lane];
+  __syncthreads();
+#pragma unroll
+  for (int j = 1; j < B; j++) {
+    if (on && r >= j) {
+      double sum = A[B * r + j][lane];
+#pragma unroll
+      for (int k = 0; k < j; k++) sum -= A[B * r + k][lane] * A[B * k + j][lane];
+      A[B * r + j][lane] = sum;
+    }
+    __syncthreads();
+    if (on && r > j) {
+      double sum = A[B * j + r][lane];
+#pragma unroll
+      for (int k = 0; k < j; k++) sum -= A[B * j + k][lane] * A[B * k + r][lane];
+      A[B * j + r][lane] = sum / A[B * j + j][lane];
+    }
+    __syncthreads();
+  }
+  if (!on) return;
+  double cv[B];
+#pragma unroll
+  for (int i = 0; i < B; i++) cv[i] = (i == r) ? 1.0 : 0.0;
+  cv[0] = cv[0] / A[0][lane];
+#pragma unroll
+  for (int i = 1; i < B; i++) {
+    double sum = cv[i];
+#pragma unroll
+    for (int k = 0; k < i; k++) sum -= A[B * i + k][lane] * cv[k];
+    cv[i] = sum / A[B * i + i][lane];
+  }
+#pragma unroll
+  for (int i = B - 2; i >= 0; i--) {
+    double sum = cv[i];
+#pragma unroll
+    for (int k = i + 1; k < B; k++) sum -= A[B * i + k][lane] * cv[k];
+    cv[i] = sum;
+  }
+  BT* Dig = (BT*)st.Dinv;
+#pragma unroll
+  for (int i = 0; i < B; i++) Dig[(size_t)(B * i + r) * N + c] = (BT)cv[i];
 }
 
 // runBackwardEulerCoupled update (JoeWithModels.cpp:4497-4517): Q += dq, then
@@ -1206,26 +1618,31 @@ void launch_turb_props(const Mesh& m, const Params& p, State& st, Turb& t, cudaS
   k_turb_cell<<<grid_for(m.ncv, TBC), TBC, 0, s>>>(m, st, t);
   k_turb_face<<<grid_for(m.nfa, TBC), TBC, 0, s>>>(m, st, t);
 }
+// HLLC: the residual, and the Jacobian blocks beside it row by row; the AUSM family forms both at once
+template <typename BT, int MODEL>
+static void launch_flux_c_m(const Mesh& m, const Params& p, State& st, Turb& t, int implicit, int for_step,
+                            cudaStream_t s) {
+  // 64-cell blocks keep the 7x7 accumulators (49 x 64 doubles) within 48 KB
+  constexpr int T = MODEL == JG_TURB_SST ? 64 : TBC;
+  const int g = grid_for(m.ncv, T);
+  const size_t shm = TM<MODEL>::BB * T * sizeof(double);
+  if (p.flux == JG_FLUX_AUSMDV || p.flux == JG_FLUX_HAENEL) {
+    if (implicit) k_flux_c<BT, MODEL, 1, true><<<g, T, shm, s>>>(m, p, st, t, for_step);
+    else k_flux_c<BT, MODEL, 1, false><<<g, T, 0, s>>>(m, p, st, t, for_step);
+    return;
+  }
+  k_flux_c<BT, MODEL, 0, false><<<g, T, 0, s>>>(m, p, st, t, for_step);
+  if (!implicit) return;
+  // FP32 blocks: the FP64 diagonal block the inverse is formed from
+  double* dfull = sizeof(BT) == 8 ? (double*)st.D : st.dfull;
+  k_jac_c<BT, MODEL><<<grid_for(m.ncv, TBJ), TBJ, 0, s>>>(m, p, st, t, for_step, dfull);
+  if (for_step) k_inv_c<BT, TM<MODEL>::B><<<grid_for(m.ncv, 32), 32 * TM<MODEL>::B, 0, s>>>(m, st, dfull);
+}
 template <typename BT>
 static void launch_flux_c_t(const Mesh& m, const Params& p, State& st, Turb& t, int implicit, int for_step,
                             cudaStream_t s) {
-  // 64-cell blocks keep the 7x7 accumulators (49 x 64 doubles) within 48 KB
-  const bool ausm = p.flux == JG_FLUX_AUSMDV || p.flux == JG_FLUX_HAENEL;
-  if (t.model == JG_TURB_SST) {
-    if (ausm)
-      k_flux_c<BT, JG_TURB_SST, 1><<<grid_for(m.ncv, 64), 64, 49 * 64 * sizeof(double), s>>>(m, p, st, t, implicit,
-                                                                                             for_step);
-    else
-      k_flux_c<BT, JG_TURB_SST, 0><<<grid_for(m.ncv, 64), 64, 49 * 64 * sizeof(double), s>>>(m, p, st, t, implicit,
-                                                                                             for_step);
-  } else {
-    if (ausm)
-      k_flux_c<BT, JG_TURB_SA, 1><<<grid_for(m.ncv, TBC), TBC, 36 * TBC * sizeof(double), s>>>(m, p, st, t,
-                                                                                              implicit, for_step);
-    else
-      k_flux_c<BT, JG_TURB_SA, 0><<<grid_for(m.ncv, TBC), TBC, 36 * TBC * sizeof(double), s>>>(m, p, st, t,
-                                                                                              implicit, for_step);
-  }
+  if (t.model == JG_TURB_SST) launch_flux_c_m<BT, JG_TURB_SST>(m, p, st, t, implicit, for_step, s);
+  else launch_flux_c_m<BT, JG_TURB_SA>(m, p, st, t, implicit, for_step, s);
 }
 void launch_flux6(const Mesh& m, const Params& p, State& st, Turb& t, int implicit, int for_step, cudaStream_t s) {
   launch_face_sensors(m, p, st, s);  // AUSMDV's shock sensor

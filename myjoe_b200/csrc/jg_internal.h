@@ -96,6 +96,7 @@ struct State {
   double* b;        // [N][5] under-relaxed rhs of the linear system
   void* D;          // [25][N] diagonal block (double or float), component-major
   void* Dinv;       // [25][N] its inverse
+  double* dfull;    // [bs^2][N] coupled path, FP32 blocks: the diagonal block in FP64, for its inverse
   void* O;          // ELL off-diagonal blocks
   void* x0;         // [5][N] relaxation vectors (double or float)
   void* x1;
