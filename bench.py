@@ -320,7 +320,7 @@ def main():
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--face-loop", default="auto", choices=["auto", "1", "2", "4", "17", "33", "34", "36", "40"],
                     help="face loop shape: autotuned; fused 1/2/4 lanes per cell or 17 (one lane, 3 blocks per SM); "
-                         "split 32 + lanes per cell of the residual kernel")
+                         "split 33, 34, 36 or 40 (one shape)")
     ap.add_argument("--converge-cases", type=int, default=24,
                     help="cases of the time-to-converge leg (0: skip it)")
     ap.add_argument("--converge-cells", default="5000,500000", help="cells log-uniform on lo,hi")
@@ -486,8 +486,8 @@ def main():
     sweep_gbs = sweep_b * n / (sweep_avg * 1e-3) / 1e9
     face_gbs = face_b * n / (face_avg * 1e-3) / 1e9
     split = tuned_cl >= 32
-    face_name = ("face loop: k_res (residual, %d lanes per cell) beside k_jac (Jacobian blocks) on a second stream"
-                 % (tuned_cl - 32) if split else "k_flux (fused face loop + Jacobian assembly)")
+    face_name = ("face loop: k_face_flux + k_res (residual) beside k_jac (Jacobian blocks) on a second stream"
+                 if split else "k_flux (fused face loop + Jacobian assembly)")
     if solve_avg >= face_avg:
         dom = {"kernel": "k_jacobi (block point-relaxation sweep)", "bound": "hbm", "achieved": sweep_gbs,
                "peak": peak, "unit": "GB/s", "frac": sweep_gbs / peak, "traffic": None,
@@ -533,8 +533,7 @@ def main():
                 "config": {"workload": WORKLOAD, "cells": n, "internal_faces_per_cell": round(f_int, 4),
                            "precision": args.precision, "l2": "flushed between timed steps (256 MB write)",
                            "parallelism": "replicas" if world > 1 else "single case",
-                           "launch_shape": {"face_loop": (("split: residual %d lanes per cell + Jacobian kernel"
-                                                           % (tuned_cl - 32)) if split else
+                           "launch_shape": {"face_loop": ("split: residual (a thread per face) + Jacobian kernel" if split else
                                                           "fused, 1 lane per cell, 3 blocks per SM" if tuned_cl == 17
                                                           else "fused, %d lanes per cell" % tuned_cl),
                                             "code": tuned_cl, "sweep_kernel": tuned_sweep}},

@@ -431,9 +431,11 @@ __device__ void grad_sdwls(const Mesh& m, const Params& p, const State& st, int 
 }
 
 // SCHEME: the gradient scheme (JG_GRAD_*) as a template parameter, so that each
-// scheme's kernel holds only its own registers
-template <int SCHEME>
-__global__ void k_grad(Mesh m, Params p, State st, int do_euler, int do_visc, int visc_lim_u, int visc_lim_h,
+// scheme's kernel holds only its own registers.  MINB: resident blocks per SM.  A thread's rows and
+// records arrive by gathers whose latency other warps cover: 137 registers leave three blocks,
+// capped at 128 (24 bytes of spills) four.  The cap pays once the grid is several waves
+template <int SCHEME, int MINB>
+__global__ void __launch_bounds__(128, MINB) k_grad(Mesh m, Params p, State st, int do_euler, int do_visc, int visc_lim_u, int visc_lim_h,
                        int separate_guv) {
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.ncv || !st.case_active[m.case_of[c]]) return;  // a frozen case keeps its arrays
@@ -1053,12 +1055,16 @@ void launch_dt(const Mesh& m, const Params& p, State& st, int use_ctrl, double c
 static void launch_grad_k(const Mesh& m, const Params& p, State& st, int do_euler, int do_visc, int lim_u, int lim_h,
                           int separate, cudaStream_t s) {
   const int g = grid_for(m.ncv, TB);
+  // least squares above seven blocks per SM (148): four resident blocks.  us, three -> four: 64 blocks
+  // 11.9 -> 12.2, 384 (viscous) 16.4 -> 17.4, 784 (viscous) 37 -> 39, 2,344 88 -> 72
   if (p.grad_scheme == JG_GRAD_GREENGAUSS)
-    k_grad<JG_GRAD_GREENGAUSS><<<g, TB, 0, s>>>(m, p, st, do_euler, do_visc, lim_u, lim_h, separate);
+    k_grad<JG_GRAD_GREENGAUSS, 1><<<g, TB, 0, s>>>(m, p, st, do_euler, do_visc, lim_u, lim_h, separate);
   else if (p.grad_scheme == JG_GRAD_SDWLS)
-    k_grad<JG_GRAD_SDWLS><<<g, TB, 0, s>>>(m, p, st, do_euler, do_visc, lim_u, lim_h, separate);
+    k_grad<JG_GRAD_SDWLS, 1><<<g, TB, 0, s>>>(m, p, st, do_euler, do_visc, lim_u, lim_h, separate);
+  else if (g > 7 * 148)
+    k_grad<JG_GRAD_LSQ, 4><<<g, TB, 0, s>>>(m, p, st, do_euler, do_visc, lim_u, lim_h, separate);
   else
-    k_grad<JG_GRAD_LSQ><<<g, TB, 0, s>>>(m, p, st, do_euler, do_visc, lim_u, lim_h, separate);
+    k_grad<JG_GRAD_LSQ, 1><<<g, TB, 0, s>>>(m, p, st, do_euler, do_visc, lim_u, lim_h, separate);
 }
 void launch_grad(const Mesh& m, const Params& p, State& st, cudaStream_t s) {
   int do_euler = p.second_order;
