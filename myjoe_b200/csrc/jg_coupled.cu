@@ -278,8 +278,8 @@ __global__ void k_turb_face(Mesh m, State st, Turb t) {
 }
 
 // ---------------------------------------------------------------------------
-// coupled HLLC flux and matrices (UgpWithCvCompFlow.cpp:1808-2289; ConvTerm =
-// 1, dp/dscal = 0); k is the kinetic energy of the state (SST), else 0
+// coupled HLLC flux (UgpWithCvCompFlow.cpp:1808-1933; ConvTerm = 1, dp/dscal = 0; its matrices are
+// formed row by row, hllc_rows_c); k is the kinetic energy of the state (SST), else 0
 // ---------------------------------------------------------------------------
 template <int NS>
 struct CState {
@@ -343,40 +343,6 @@ __device__ void flux_hllc_c(double* F, const CState<NS>& L, const CState<NS>& R,
   for (int i = 0; i < B; i++) F[i] *= area;
 }
 
-// calcJacobianCoupled_HLLC (:2180-2244); nA = n * area
-template <int NS>
-__device__ void jac_c(double* A, const double* vel, double pp, double rrho, double hh, const double* sc,
-                      const double* nA, double gamma) {
-  constexpr int B = 5 + NS;
-  double kapm1 = gamma - 1.0;
-  double nVel[3] = {vel[0] * nA[0], vel[1] * nA[1], vel[2] * nA[2]};
-  double U_k = nVel[0] + nVel[1] + nVel[2];
-  double vSquHlf = 0.5 * dot3(vel, vel);
-  A[0] = 0.0; A[1] = nA[0]; A[2] = nA[1]; A[3] = nA[2]; A[4] = 0.0;
-  for (int s = 0; s < NS; s++) A[5 + s] = 0.0;
-  for (int r = 0; r < 3; r++) {
-    double* a = A + B * (1 + r);
-    a[0] = -vel[r] * U_k + nA[r] * (kapm1 * vSquHlf + gamma * pp / rrho - kapm1 * hh);
-    for (int c = 0; c < 3; c++)
-      a[1 + c] = (r == c) ? (2.0 - gamma) * nVel[r] + U_k : vel[r] * nA[c] - kapm1 * vel[c] * nA[r];
-    a[4] = kapm1 * nA[r];
-    for (int s = 0; s < NS; s++) a[5 + s] = 0.0 * nA[r];
-  }
-  double* a4 = A + 4 * B;
-  a4[0] = U_k * ((gamma - 2.0) * vSquHlf - gamma * (hh - pp / rrho));
-  for (int c = 0; c < 3; c++) a4[1 + c] = (hh + vSquHlf) * nA[c] - kapm1 * vel[c] * U_k;
-  a4[4] = gamma * U_k;
-  for (int s = 0; s < NS; s++) a4[5 + s] = 0.0 * U_k;
-  for (int s = 0; s < NS; s++) {
-    double* a = A + B * (5 + s);
-    a[0] = 0.0;
-    for (int c = 0; c < 3; c++) a[1 + c] = sc[s] * nA[c];
-    a[4] = 0.0;
-    for (int q = 0; q < NS; q++) a[5 + q] = 0.0;
-    a[5 + s] = rrho * U_k;
-  }
-}
-
 // calcdSMdU_HLLC (:2247-2266)
 template <int NS>
 __device__ void dsmdu_c(double* d, const double* vel, double pp, double rrho, double hh, const double* nV,
@@ -388,132 +354,6 @@ __device__ void dsmdu_c(double* d, const double* vel, double pp, double rrho, do
   for (int i = 0; i < 3; i++) d[1 + i] = Factor * invertrho * ((2 * U_k - S - SM) * nV[i] - kapm1 * vel[i]);
   d[4] = Factor * invertrho * kapm1;
   for (int s = 0; s < NS; s++) d[5 + s] = Factor * invertrho * 0.0;
-}
-
-// calcSubSonicJacobianCoupled_HLLC (:2270-2289)
-template <int NS>
-__device__ void subsonic_c(double* A, const double* d, double rhoS, const double* rhouS, double rhoeS,
-                           const double* sc, double pS, double Om, double sM, double rhoSmq, const double* nV,
-                           double area) {
-  constexpr int B = 5 + NS;
-  double OmSM = Om * sM, OmSMp1 = OmSM + 1.0;
-  double rr[B];
-  rr[0] = rhoS;
-  for (int i = 0; i < 3; i++) rr[1 + i] = rhouS[i] + rhoSmq * nV[i];
-  rr[4] = rhoeS + pS + rhoSmq * sM;
-  for (int s = 0; s < NS; s++) rr[5 + s] = rhoS * sc[s];
-  for (int i = 0; i < B; i++)
-    for (int r = 0; r < B; r++) A[B * r + i] = -OmSM * A[B * r + i] + area * OmSMp1 * d[i] * rr[r];
-}
-
-// calcEulerFluxMatricesCoupled_HLLC (:1934-2176), then dU/dQ of the scalar columns
-template <int NS>
-__device__ void matrices_hllc_c(double* AL, double* AR, const CState<NS>& L, const CState<NS>& R, double area,
-                                const double* nV, bool only_p) {
-  constexpr int B = 5 + NS, BB = B * B;
-  if (!only_p) {
-    double dd[B];
-    double unL = dot3(L.u, nV), uLuL = dot3(L.u, L.u), cL = sqrt(L.gam * L.p / L.rho);
-    double hL = L.h + L.k, rhoeL = (hL + 0.5 * uLuL) * L.rho - L.p;
-    double unR = dot3(R.u, nV), uRuR = dot3(R.u, R.u), cR = sqrt(R.gam * R.p / R.rho);
-    double hR = R.h + R.k, rhoeR = (hR + 0.5 * uRuR) * R.rho - R.p;
-    double Rrho = sqrt(R.rho / L.rho);
-    double tmp = 1.0 / (1.0 + Rrho);
-    double vR[3];
-    for (int i = 0; i < 3; i++) vR[i] = tmp * (L.u[i] + R.u[i] * Rrho);
-    double uRoe = dot3(vR, nV);
-    double gpr = tmp * ((L.gam * L.p / L.rho + 0.5 * (L.gam - 1.0) * uLuL) +
-                        (R.gam * R.p / R.rho + 0.5 * (R.gam - 1.0) * uRuR) * Rrho);
-    double cRoe = sqrt(gpr - ((L.gam + R.gam) * 0.5 - 1.0) * 0.5 * dot3(vR, vR));
-    double sL = fmin(uRoe - cRoe, unL - cL);
-    double sR = fmax(uRoe + cRoe, unR + cR);
-    double invrhotld = 1.0 / (R.rho * (sR - unR) - L.rho * (sL - unL));
-    double sM = (L.p - R.p - L.rho * unL * (sL - unL) + R.rho * unR * (sR - unR)) /
-                (R.rho * (sR - unR) - L.rho * (sL - unL));
-    double pS = R.rho * (unR - sR) * (unR - sM) + R.p;
-    double nA[3] = {nV[0] * area, nV[1] * area, nV[2] * area};
-    if (sM >= 0.0) {
-      if (sL > 0.0) {
-        if (AL) jac_c<NS>(AL, L.u, L.p, L.rho, hL, L.sc, nA, L.gam);
-        if (AR)
-          for (int e = 0; e < BB; e++) AR[e] = 0.0;
-      } else {
-        double Om = 1.0 / (sL - sM), d = sL - unL;
-        double rhoS = L.rho * d * Om, rhouS[3];
-        for (int i = 0; i < 3; i++) rhouS[i] = (L.rho * L.u[i] * d + (pS - L.p) * nV[i]) * Om;
-        double rhoeS = (d * rhoeL - L.p * unL + pS * sM) * Om;
-        if (AL) {
-          dsmdu_c<NS>(dd, L.u, L.p, L.rho, hL, nV, L.gam, sM, sL, invrhotld, 1.0);
-          jac_c<NS>(AL, L.u, L.p, L.rho, hL, L.sc, nA, L.gam);
-          subsonic_c<NS>(AL, dd, rhoS, rhouS, rhoeS, L.sc, pS, Om, sM, R.rho * (sR - unR), nV, area);
-          for (int i = 0; i < 5; i++) AL[(B + 1) * i] += area * Om * sM * sL;
-          for (int s = 0; s < NS; s++) {
-            AL[(5 + s) * B] += area * Om * sM * sL * L.sc[s];
-            AL[(5 + s) * B + 5 + s] += area * Om * sM * sL * L.rho;
-          }
-        }
-        if (AR) {
-          dsmdu_c<NS>(dd, R.u, R.p, R.rho, hR, nV, R.gam, sM, sR, invrhotld, -1.0);
-          for (int e = 0; e < BB; e++) AR[e] = 0.0;
-          subsonic_c<NS>(AR, dd, rhoS, rhouS, rhoeS, L.sc, pS, Om, sM, L.rho * (sL - unL), nV, area);
-        }
-      }
-    } else {
-      if (sR >= 0.0) {
-        double Om = 1.0 / (sR - sM), d = sR - unR;
-        double rhoS = R.rho * d * Om, rhouS[3];
-        for (int i = 0; i < 3; i++) rhouS[i] = (R.rho * R.u[i] * d + (pS - R.p) * nV[i]) * Om;
-        double rhoeS = (d * rhoeR - R.p * unR + pS * sM) * Om;
-        if (AR) {
-          dsmdu_c<NS>(dd, R.u, R.p, R.rho, hR, nV, R.gam, sM, sR, invrhotld, -1.0);
-          jac_c<NS>(AR, R.u, R.p, R.rho, hR, R.sc, nA, R.gam);
-          subsonic_c<NS>(AR, dd, rhoS, rhouS, rhoeS, R.sc, pS, Om, sM, L.rho * (sL - unL), nV, area);
-          for (int i = 0; i < 5; i++) AR[(B + 1) * i] += area * Om * sM * sR;
-          for (int s = 0; s < NS; s++) {
-            AR[(5 + s) * B] += area * Om * sM * sR * R.sc[s];
-            AR[(5 + s) * B + 5 + s] += area * Om * sM * sR * R.rho;
-          }
-        }
-        if (AL) {
-          dsmdu_c<NS>(dd, L.u, L.p, L.rho, hL, nV, L.gam, sM, sL, invrhotld, 1.0);
-          for (int e = 0; e < BB; e++) AL[e] = 0.0;
-          subsonic_c<NS>(AL, dd, rhoS, rhouS, rhoeS, R.sc, pS, Om, sM, R.rho * (sR - unR), nV, area);
-        }
-      } else {
-        if (AR) jac_c<NS>(AR, R.u, R.p, R.rho, hR, R.sc, nA, R.gam);
-        if (AL)
-          for (int e = 0; e < BB; e++) AL[e] = 0.0;
-      }
-    }
-  } else {
-    if (AL) {
-      double uLuL = dot3(L.u, L.u), hL = L.h + L.k, g = L.gam;
-      for (int j = 0; j < B; j++) AL[j] = 0.0;
-      double dpdrho = 0.5 * (g - 1.0) * uLuL - (g - 1.0) * hL + g * L.p / L.rho;
-      for (int r = 0; r < 3; r++) {
-        double* a = AL + B * (1 + r);
-        a[0] = dpdrho * nV[r] * area;
-        for (int c = 0; c < 3; c++) a[1 + c] = -(g - 1.0) * L.u[c] * nV[r] * area;
-        a[4] = (g - 1.0) * nV[r] * area;
-        for (int s = 0; s < NS; s++) a[5 + s] = 0.0 * nV[r] * area;
-      }
-      for (int e = 4 * B; e < BB; e++) AL[e] = 0.0;
-    }
-    if (AR)
-      for (int e = 0; e < BB; e++) AR[e] = 0.0;
-  }
-  if (AL)
-    for (int j = 0; j < B; j++)
-      for (int s = 0; s < NS; s++) {
-        AL[B * j] -= L.sc[s] / L.rho * AL[B * j + 5 + s];
-        AL[B * j + 5 + s] /= L.rho;
-      }
-  if (AR)
-    for (int j = 0; j < B; j++)
-      for (int s = 0; s < NS; s++) {
-        AR[B * j] -= R.sc[s] / R.rho * AR[B * j + 5 + s];
-        AR[B * j + 5 + s] /= R.rho;
-      }
 }
 
 // ---------------------------------------------------------------------------
@@ -661,13 +501,6 @@ __device__ __forceinline__ void cflux(double* F, const CState<NS>& L, const CSta
   if (FK == 0) flux_hllc_c<NS>(F, L, R, area, nV, only_p);
   else flux_ausm_c<NS>(F, L, R, area, nV, only_p, haenel, fo);
 }
-template <int NS, int FK>
-__device__ __forceinline__ void cmatrices(double* AL, double* AR, const CState<NS>& L, const CState<NS>& R,
-                                          double area, const double* nV, bool only_p, bool haenel, int fo) {
-  if (FK == 0) matrices_hllc_c<NS>(AL, AR, L, R, area, nV, only_p);
-  else matrices_ausm_c<NS>(AL, AR, L, R, area, nV, only_p, haenel, fo);
-}
-
 // ---------------------------------------------------------------------------
 // calcViscousFluxCoupled (UgpWithCvCompFlow.cpp:3040-3276) with the model's k
 // ---------------------------------------------------------------------------
@@ -965,7 +798,7 @@ __device__ __forceinline__ void model_source(const Mesh& m, const State& st, con
 // IMPL: with the Jacobian blocks (the AUSM family); else the residual alone
 template <typename BT, int MODEL, int FK, bool IMPL>
 __global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb t, int for_step) {
-  constexpr bool implicit = IMPL;
+  static_assert(!IMPL || FK == 1, "HLLC forms its blocks in k_jac_c");
   constexpr int NS = TM<MODEL>::NS, B = TM<MODEL>::B, BB = TM<MODEL>::BB;
   constexpr bool SST = MODEL == JG_TURB_SST;
   extern __shared__ double sD[];  // [BB][blockDim.x]
@@ -976,7 +809,7 @@ __global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb
   const bool only_p = p.symm_bc == JG_SYMM_ANALYTICAL;
   double rhs[B];
   for (int i = 0; i < B; i++) rhs[i] = 0.0;
-  if (implicit)
+  if constexpr (IMPL)
     for (int e = 0; e < BB; e++) sD[e * bd + tid] = 0.0;
   BT* O = (BT*)st.O;
   double F[B];
@@ -1004,10 +837,10 @@ __global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb
         for (int i = 0; i < B; i++) rhs[i] += sg * F[i];
       }
       double Ob[BB];
-      if (implicit) {
+      if constexpr (IMPL) {
         CState<NS> L0 = cell_c<NS>(m, p, st, t, c0, SST), R0 = cell_c<NS>(m, p, st, t, c1, SST);
         double Apl[BB], Ami[BB];
-        cmatrices<NS, FK>(Apl, Ami, L0, R0, area, nV, false, hz, fo);
+        matrices_ausm_c<NS>(Apl, Ami, L0, R0, area, nV, false, hz, fo);
         // row of c0: D += Apl, O = Ami ; row of c1: D -= Ami, O = -Apl
         if (s.side == 0) {
           for (int e = 0; e < BB; e++) { sD[e * bd + tid] += Apl[e]; Ob[e] = Ami[e]; }
@@ -1035,7 +868,7 @@ __global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb
         visc_flux_c<NS>(F, vf, v0, v1, st.mul_fa[f], st.mut_fa[f], st.lam_fa[f], p.PrTurb, kine_fa, ufa, dfa, one,
                         area, nV, smag, sV, alpha);
         for (int i = 0; i < B; i++) rhs[i] += sg * F[i];
-        if (implicit) {
+        if constexpr (IMPL) {
           // row of c0: D += A0, O += A1 ; row of c1: D -= A1, O -= A0  (JoeWithModels.cpp:5110-5127)
           double Dv[BB];
           for (int e = 0; e < BB; e++) Dv[e] = 0.0;
@@ -1049,7 +882,7 @@ __global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb
           for (int e = B; e < BB; e++) sD[e * bd + tid] += Dv[e];
         }
       }
-      if (implicit)
+      if constexpr (IMPL)
         for (int e = 0; e < BB; e++) O[ell_c<BB>(m, c, s.col, e)] = (BT)Ob[e];
     } else {
       // boundary face; the cell is cvofa[f][0] (JoeWithModels.cpp:5139-5799)
@@ -1062,14 +895,14 @@ __global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb
         const bool op = (z.kind == JG_BC_SYMMETRY) && only_p;
         cflux<NS, FK>(F, Bs, Bs, area, nV, op, hz_b, fob);
         for (int i = 0; i < B; i++) rhs[i] -= F[i];
-        if (implicit) {
+        if constexpr (IMPL) {
           if (z.kind == JG_BC_NEUMANN || p.symm_bc == JG_SYMM_NEW_NUMERIC) {
             double Apl[BB], Ami[BB];
-            cmatrices<NS, FK>(Apl, Ami, Bs, Bs, area, nV, false, hz_b, fob);
+            matrices_ausm_c<NS>(Apl, Ami, Bs, Bs, area, nV, false, hz_b, fob);
             for (int e = 0; e < BB; e++)
               sD[e * bd + tid] += (p.symm_bc == JG_SYMM_NEW_NUMERIC) ? Apl[e] + Ami[e] : Apl[e];
           } else {
-            cmatrices<NS, FK>(Dv, nullptr, Bs, Bs, area, nV, only_p, hz_b, fob);
+            matrices_ausm_c<NS>(Dv, nullptr, Bs, Bs, area, nV, only_p, hz_b, fob);
             for (int e = 0; e < BB; e++) sD[e * bd + tid] += Dv[e];
           }
         }
@@ -1088,7 +921,7 @@ __global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb
           visc_flux_c<NS>(F, vf, vb, vb, st.mul_fa[f], st.mut_fa[f], st.lam_fa[f], p.PrTurb, Bs.k, vb.u, dfa, one,
                           area, nV, smag, nV, 1.0);
           for (int i = 0; i < B; i++) rhs[i] -= F[i];
-          if (implicit) {
+          if constexpr (IMPL) {
             for (int e = 0; e < BB; e++) Dv[e] = 0.0;
             visc_jac_c_add<NS>(Dv, 1.0, 0, vf, vb, vb.u, p.R, area);
             for (int e = B; e < BB; e++) sD[e * bd + tid] += Dv[e];
@@ -1098,13 +931,13 @@ __global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb
         // the wall keeps the face kinetic energy at 0 (JoeWithModels.cpp:5448-5452)
         cflux<NS, FK>(F, Bs, Bs, area, nV, only_p, hz_b, fob);
         for (int i = 0; i < B; i++) rhs[i] -= F[i];
-        if (implicit) {
+        if constexpr (IMPL) {
           if (p.symm_bc == JG_SYMM_NEW_NUMERIC) {
             double Apl[BB], Ami[BB];
-            cmatrices<NS, FK>(Apl, Ami, Bs, Bs, area, nV, false, hz_b, fob);
+            matrices_ausm_c<NS>(Apl, Ami, Bs, Bs, area, nV, false, hz_b, fob);
             for (int e = 0; e < BB; e++) sD[e * bd + tid] += Apl[e] + Ami[e];
           } else {
-            cmatrices<NS, FK>(Dv, nullptr, Bs, Bs, area, nV, only_p, hz_b, fob);
+            matrices_ausm_c<NS>(Dv, nullptr, Bs, Bs, area, nV, only_p, hz_b, fob);
             for (int e = 0; e < BB; e++) sD[e * bd + tid] += Dv[e];
           }
         }
@@ -1121,7 +954,7 @@ __global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb
         visc_flux_c<NS>(F, vf, v0, vb, st.mul_fa[f], 0.0, st.lam_fa[f], p.PrTurb, 0.0, vb.u, dfa, dterm, area, nV,
                         smag, nV, 1.0);
         for (int i = 0; i < B; i++) rhs[i] -= F[i];
-        if (implicit) {
+        if constexpr (IMPL) {
           for (int e = 0; e < BB; e++) Dv[e] = 0.0;
           visc_jac_c_add<NS>(Dv, 1.0, 0, vf, v0, vb.u, p.R, area);
           for (int e = B; e < BB; e++) sD[e * bd + tid] += Dv[e];
@@ -1132,9 +965,9 @@ __global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb
         if (SST) Bs.k = Bs.sc[0];
         cflux<NS, FK>(F, L, Bs, area, nV, false, hz_b, fob);
         for (int i = 0; i < B; i++) rhs[i] -= F[i];
-        if (implicit) {
+        if constexpr (IMPL) {
           CState<NS> L0 = cell_c<NS>(m, p, st, t, c, SST);
-          cmatrices<NS, FK>(Dv, nullptr, L0, Bs, area, nV, false, hz_b, fob);
+          matrices_ausm_c<NS>(Dv, nullptr, L0, Bs, area, nV, false, hz_b, fob);
           for (int e = 0; e < BB; e++) sD[e * bd + tid] += Dv[e];
         }
         VSideC<NS> v0 = vcell_c<NS>(m, st, t, p, c, SST);
@@ -1154,7 +987,7 @@ __global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb
         visc_flux_c<NS>(F, vf, v0, vb, st.mul_fa[f], st.mut_fa[f], st.lam_fa[f], p.PrTurb, Bs.k, vb.u, dfa, dterm,
                         area, nV, smag, sV, alpha);
         for (int i = 0; i < B; i++) rhs[i] -= F[i];
-        if (implicit) {
+        if constexpr (IMPL) {
           for (int e = 0; e < BB; e++) Dv[e] = 0.0;
           visc_jac_c_add<NS>(Dv, 1.0, 0, vf, v0, vb.u, p.R, area);
           for (int e = B; e < BB; e++) sD[e * bd + tid] += Dv[e];
@@ -1168,7 +1001,7 @@ __global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb
   for (int i = 0; i < B; i++) st.rhs[(size_t)B * c + i] = rhs[i];
   if (for_step)
     for (int i = 0; i < B; i++) st.b[(size_t)B * c + i] = p.under_relax * rhs[i];
-  if (implicit) {
+  if constexpr (IMPL) {
     double Dm[BB];
     for (int e = 0; e < BB; e++) Dm[e] = sD[e * bd + tid];
     gravity_diag<B>(p, m, c, Dm);
@@ -1192,10 +1025,11 @@ __global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb
 // The Jacobian blocks with HLLC, row by row: every row of a face's two matrices goes into the cell's
 // diagonal block (shared memory) and its off-diagonal block as soon as it is formed, so no thread
 // holds a B x B matrix.  Formed whole beside the residual, the matrices cost 255 registers, spills
-// and two blocks per SM (100k cells 6x6 FP64: 429 us for both -> 71 residual + 197 here + 24 inverse; 7x7
-// FP32 393 -> 88 + 133 + 24 at 70k; capped at 168 registers the rows spill: 250 and 220).  Each entry is the expression of
-// matrices_hllc_c; of the scalars' columns only the diagonal entries differ from zero (dp/dscal = 0),
-// so the dU/dQ products with the others are left out.
+// and two blocks per SM (100k cells 6x6 FP64: 429 us for both -> 71 residual + 197 here + 24 inverse;
+// 7x7 FP32 393 -> 88 + 133 + 24 at 70k; capped at 168 registers the rows spill: 250 and 220).  Each
+// entry is calcEulerFluxMatricesCoupled_HLLC's (UgpWithCvCompFlow.cpp:1934-2289); of the scalars'
+// columns only the diagonal entries differ from zero (dp/dscal = 0), so the dU/dQ products with the
+// others are left out.
 // ---------------------------------------------------------------------------
 // emit(r, aL, aR): rows r of A_L and A_R
 template <int NS, typename Emit>
