@@ -1089,7 +1089,10 @@ void launch_grad_coupled(const Mesh& m, const Params& p, State& st, cudaStream_t
 }
 // both sweep kernels do the same arithmetic in the same order (bit-identical results)
 void launch_jacobi(const Mesh& m, const Params& p, State& st, int sweeps, cudaStream_t s) {
-  if (p.relax_variant != 1) {
+  // FP32 rows stream better a cell per thread once the matrix is well above L2 (us per ten sweeps, slice
+  // kernel / this one: 100k cells 109 / 129, 250k 344 / 326, 700k 938 / 867); the bits are the same
+  const bool cells = p.relax_variant == 1 || (p.fp32 && m.nslices > 5000);
+  if (!cells) {
     if (p.fp32) sweep_jacobi<float, 5>(m, st, sweeps, s);
     else sweep_jacobi<double, 5>(m, st, sweeps, s);
     return;

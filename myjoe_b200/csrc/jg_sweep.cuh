@@ -17,7 +17,7 @@
 //    may not be seen by a later one that started before the boundary.
 // Measured, 10 sweeps, the loop over one column at a time before -> now: 8k cells FP64 Jacobi 61 ->
 // 35 us, 50k 84 -> 82, 250k 576 -> 535, 700k 1485 -> 1405 (5.8 -> 6.2 TB/s of matrix); FP32 8k 49 ->
-// 23, 250k 391 -> 344, 700k 1004 -> 938.
+// 23; FP32 SGS 250k 299 -> 264 (20 passes -> 11 besides).
 //
 // Every sum keeps its order (k within a column, column by column), so the results are bit for bit
 // those of the thread-per-cell kernel (k_jacobi).
@@ -144,7 +144,7 @@ int resident_blocks(void (*kernel)(P...), int block) {
 // One pass.  A grid that fits the GPU in one wave takes the widest chunk of columns (the shortest
 // dependent chain); a larger FP64 grid lives on resident blocks instead, so it takes three columns
 // while those blocks fit one wave and one column with all 2,048 threads of an SM above.  FP32 rows
-// are half as wide in registers and take the whole row at any size.  Us per solve (10 sweeps; FP64
+// are half as wide in registers and take the whole row at any size (packed above one wave).  Us per solve (10 sweeps; FP64
 // Jacobi 8k / 35k / 50k / 250k / 700k cells): six columns 35 / 82 / 117 / 754 / 2012, three 37 / 55 /
 // 94 / 563 / 1487, one 43 / 76 / 82 / 535 / 1405; FP32 SGS 8k / 50k / 250k / 700k: six 25 / 41 / 242 /
 // 634, three 35 / 49 / 272 / 693, one 47 / 64 / 291 / 704.
@@ -153,13 +153,13 @@ void launch_sweep(const Mesh& m, const State& st, int grid, const BT* xin, BT* x
                   const int* slices, bool after_pass, cudaStream_t s) {
   constexpr int T = B * SLICE;
   auto wide = k_sweep<BT, B, KIND, SWEEP_COLS, 1>;
+  // FP32 above one wave: registers for 960 threads per SM (left to itself the compiler takes 80 a thread:
+  // 250k cells SGS 320 us a solve, capped 264; below one wave the uncapped kernel is 3% faster)
+  auto packed = k_sweep<BT, B, KIND, SWEEP_COLS, sizeof(BT) == 4 ? 960 / T : 1>;
   auto mid = k_sweep<BT, B, KIND, 3, 1280 / T>;
   auto narrow = k_sweep<BT, B, KIND, 1, 1920 / T>;
-  auto kernel = wide;
-  if (sizeof(BT) == 8) {
-    static const int fit_wide = resident_blocks(wide, T), fit_mid = resident_blocks(mid, T);
-    kernel = grid <= fit_wide ? wide : grid <= fit_mid ? mid : narrow;
-  }
+  static const int fit_wide = resident_blocks(wide, T), fit_mid = resident_blocks(mid, T);
+  auto kernel = grid <= fit_wide ? wide : sizeof(BT) == 4 ? packed : grid <= fit_mid ? mid : narrow;
   if (first) kernel = narrow;  // no matrix rows to request: Dinv b
   launch_pass(kernel, grid, T, after_pass, s, m, st, xin, xout, (int)first, color, slices, nullptr, nullptr, nullptr,
               nullptr);
