@@ -191,14 +191,22 @@ static int download_rows(jg_case* h, const double* dev, double* host, const std:
   return JG_OK;
 }
 
-// the same for w doubles at the front of each device record of `stride` doubles
+// the same for w doubles at the front of each device record of `stride` doubles.  A kernel packs them
+// into the state staging, as many records at a time as it holds, and each lot is one copy: a strided
+// copy into pageable memory goes row by row (250k cells, the four gradients: 145 ms against 2.2 ms)
 static int download_fields(jg_case* h, const double* dev, size_t stride, double* host, const std::vector<int>& perm,
                            size_t n, size_t w) {
   std::vector<double> tmp(perm.empty() ? 0 : n * w);
   double* to = perm.empty() ? host : tmp.data();
-  if (n)
-    CK(cudaMemcpy2DAsync(to, w * sizeof(double), dev, stride * sizeof(double), w * sizeof(double), n,
-                         cudaMemcpyDeviceToHost, h->stream));
+  if (!h->d_io) RC(dmalloc(h, &h->d_io, 5 * (size_t)h->ncv));
+  // records a lot (an allocation is at least 256 bytes: one cell's fields fit)
+  const size_t lot = alloc_round(5 * (size_t)h->ncv * sizeof(double)) / sizeof(double) / w;
+  for (size_t c = 0; c < n; c += lot) {
+    const size_t k = std::min(lot, n - c);
+    launch_pack_fields(k, w, stride, dev + c * stride, h->d_io, h->stream);
+    CKL();
+    CK(cudaMemcpyAsync(to + c * w, h->d_io, k * w * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+  }
   CK(cudaStreamSynchronize(h->stream));
   if (!perm.empty()) rows_to_caller(perm, tmp.data(), host, n, w, 1);
   return JG_OK;

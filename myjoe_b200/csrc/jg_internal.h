@@ -229,6 +229,7 @@ void launch_flux_faces(int kind, int n, const double* L, const double* R, const 
 // io ([5][n] planes rho, rhou, rhoE) <-> q ([n][5]); perm (or nullptr): the io row of each cell
 void launch_pack_state(int n, const double* io, double* q, const int* perm, cudaStream_t s);
 void launch_unpack_state(int n, const double* q, double* io, const int* perm, cudaStream_t s);
+void launch_pack_fields(size_t n, size_t w, size_t stride, const double* rec, double* io, cudaStream_t s);
 
 int grid_for(long n, int block);
 int record_error(int code, const char* msg);  // sets the jg_last_error message

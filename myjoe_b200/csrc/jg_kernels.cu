@@ -982,6 +982,14 @@ void launch_pack_state(int n, const double* io, double* q, const int* perm, cuda
 void launch_unpack_state(int n, const double* q, double* io, const int* perm, cudaStream_t s) {
   k_unpack_state<<<grid_for(n, 256), 256, 0, s>>>(n, q, io, perm);
 }
+// w doubles at the front of each record of `stride` doubles, packed (jg_get_gradients)
+__global__ void k_pack_fields(size_t total, int w, int stride, const double* rec, double* io) {
+  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (i < total) io[i] = rec[i / w * stride + i % w];
+}
+void launch_pack_fields(size_t n, size_t w, size_t stride, const double* rec, double* io, cudaStream_t s) {
+  k_pack_fields<<<(unsigned)((n * w + 255) / 256), 256, 0, s>>>(n * w, (int)w, (int)stride, rec, io);
+}
 constexpr int TB = 128;
 
 // static face geometry, once per mesh: the unit normal and area of every face; for internal
