@@ -62,7 +62,7 @@ struct jg_case {
   int hist_cap = 0;
   double* d_tmp = nullptr;  // BiCGSTAB work vectors (8 x 5N)
   double* d_red = nullptr;  // its reductions' partial sums and scalars
-  int* bicg_flag = nullptr;  // page-locked: iteration count and stop flag of the running solve
+  unsigned long long* bicg_word = nullptr;  // page-locked: iteration count and stop flag of the running solve
   cudaEvent_t bicg_ev[2] = {nullptr, nullptr};
   cudaGraphExec_t graph = nullptr;
   int graph_sweeps = -1;
@@ -384,7 +384,7 @@ int jg_destroy(jg_case_t* h) {
   if (h->st.ev_fork) cudaEventDestroy(h->st.ev_fork);
   if (h->st.ev_join) cudaEventDestroy(h->st.ev_join);
   if (h->hpin) cudaFreeHost(h->hpin);
-  if (h->bicg_flag) cudaFreeHost(h->bicg_flag);
+  if (h->bicg_word) cudaFreeHost(h->bicg_word);
   for (cudaEvent_t e : h->bicg_ev)
     if (e) cudaEventDestroy(e);
   if (h->st.ev_pre) cudaEventDestroy(h->st.ev_pre);
@@ -1445,27 +1445,29 @@ static int bcgstab(jg_case* h, double* phi, const double* rhs, double zeroAbs, d
   const size_t n5 = 5 * (size_t)h->ncv;
   if (!h->d_tmp) RC(dmalloc(h, &h->d_tmp, 8 * n5));
   if (!h->d_red) RC(dmalloc(h, &h->d_red, 2048 + 16));
-  if (!h->bicg_flag) CK(cudaHostAlloc(&h->bicg_flag, 2 * sizeof(int), cudaHostAllocDefault));
+  if (!h->bicg_word) CK(cudaHostAlloc(&h->bicg_word, sizeof(*h->bicg_word), cudaHostAllocDefault));
   for (cudaEvent_t& e : h->bicg_ev)
     if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   double* w = h->d_tmp;
   Bicg q{phi, w, w + n5, w + 2 * n5, w + 3 * n5, w + 4 * n5, w + 5 * n5, w + 6 * n5, w + 7 * n5, h->d_red,
-         h->d_red + 2048, rhs, zeroAbs, zeroRel, maxiter, h->bicg_flag};
+         h->d_red + 2048, rhs, zeroAbs, zeroRel, maxiter, h->bicg_word};
   cudaStream_t S = h->stream;
-  h->bicg_flag[0] = h->bicg_flag[1] = 0;
+  *h->bicg_word = 0;
   CK(cudaMemsetAsync(q.p, 0, 2 * n5 * sizeof(double), S));  // p and v
   if (lines) launch_line_factor(h->m, h->st, h->lines, S);  // the lines' elimination, once per solve
   launch_bicg_start(h->m, h->st, q, S);
-  volatile int* flag = h->bicg_flag;
+  volatile unsigned long long* word = h->bicg_word;
+  unsigned long long w64 = 0;
   for (int k = 0;; k++) {
     launch_bicg_iteration(h->m, h->st, q, lines ? &h->lines : nullptr, S);
     CKL();
     CK(cudaEventRecord(h->bicg_ev[k % 2], S));
     if (k == 0) continue;
     CK(cudaEventSynchronize(h->bicg_ev[(k - 1) % 2]));
-    if (flag[1]) break;
+    w64 = *word;  // one load of both: the iteration in flight may store them meanwhile
+    if (w64 >> 32) break;
   }
-  if (iters) *iters = flag[0];  // the iteration enqueued past the stop left the count as it was
+  if (iters) *iters = (int)(w64 & 0xffffffffu);
   return JG_OK;
 }
 

@@ -141,7 +141,7 @@ template <bool RES>
 __global__ void __launch_bounds__(5 * SLICE, 8) k_bicg_spmv(Mesh m, State st, const double* x, double* y,
                                                             const double* rhs, double* y2, double* sc,
                                                             int first, double zabs, double zrel, int maxiter,
-                                                            volatile int* flag) {
+                                                            volatile unsigned long long* word) {
   constexpr int COLS = 2;
   __shared__ double xs[COLS][5][SLICE];
   __shared__ double wmax[5];
@@ -225,8 +225,7 @@ __global__ void __launch_bounds__(5 * SLICE, 8) k_bicg_spmv(Mesh m, State st, co
   sc[S_ITER] = iter;
   const bool stop = (r <= zabs) || (r / (sc[S_RES0MAX] + 1.0E-12) <= zrel) || iter > maxiter;
   if (stop) sc[S_DONE] = 1.0;
-  flag[0] = (int)iter;
-  if (stop) flag[1] = 1;
+  *word = (unsigned long long)stop << 32 | (unsigned)iter;
   __threadfence_system();
 }
 
@@ -259,7 +258,7 @@ void launch_bicg_iteration(const Mesh& m, const State& st, const Bicg& q, const 
   launch_pass(k_bicg_dot<DOT_OMEGA>, gd, RT, true, s, n5, q.s, q.t, q.part, q.sc);
   launch_pass(k_bicg_vec<VEC_PHI>, g, TB, true, s, m, st, q.sc, 1.0, q.phi, q.phat, q.shat, nullptr, 0);
   launch_pass(k_bicg_spmv<true>, m.nslices, B, true, s, m, st, q.phi, q.res, q.rhs, nullptr, q.sc, 0, q.zabs, q.zrel,
-              q.maxiter, q.flag);
+              q.maxiter, q.word);
 }
 
 }  // namespace jg

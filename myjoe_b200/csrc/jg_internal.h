@@ -299,14 +299,15 @@ void launch_line_relax(const Mesh& m, const Params& p, State& st, const Lines& L
                        cudaStream_t s);
 
 // one BiCGSTAB solve (jg_bicgstab.cu): vectors [5][N], the partial sums of the reductions (2,048
-// doubles), 16 doubles of device scalars, and the host's view of the iteration count and the stop
-// flag (page-locked, two ints)
+// doubles), 16 doubles of device scalars, and the host's view of the iteration count (low half) and
+// the stop flag (high half): one page-locked word, so that the host never reads the flag of one
+// iteration beside the count of another
 struct Bicg {
   double *phi, *res, *res0, *p, *v, *t, *s, *phat, *shat, *part, *sc;
   const double* rhs;
   double zabs, zrel;
   int maxiter;
-  volatile int* flag;
+  volatile unsigned long long* word;
 };
 void launch_bicg_start(const Mesh& m, const State& st, const Bicg& q, cudaStream_t s);
 void launch_bicg_iteration(const Mesh& m, const State& st, const Bicg& q, const Lines* lines, cudaStream_t s);

@@ -75,3 +75,24 @@ def test_iteration_limit(max_iter):
     np.testing.assert_array_equal(x, y)
     _, it = j.solveCoupledLinSysNS(A, b, 1e30, 0.0, max_iter)    # met at once
     assert it == 1
+
+
+def test_reported_count_is_that_of_the_stopping_iteration():
+    """the host reads the count while the iteration after the one it waited for may be running: with
+    every threshold and again and again, the count is that of the iteration that met it"""
+    g, prm, A, b = _system((11, 3, 1), 0, np.random.default_rng(5))
+    j = solver.JoeGpu(g, prm)
+    Di = np.linalg.inv(A[g.nbocv_i[:-1]])
+    M = scipy.sparse.bsr_matrix((A, g.nbocv_v, g.nbocv_i), shape=(5 * g.ncv, 5 * g.ncv)).tocsr()
+
+    def norm(x):
+        r = b - (M @ x.ravel()).reshape(-1, 5)
+        return np.abs(np.einsum("nij,nj->ni", Di, r)).max()
+    n = [norm(np.zeros_like(b))] + [norm(j.solveCoupledLinSysNS(A, b, -1.0, -1.0, k)[0]) for k in range(6)]
+    for k in range(1, 7):
+        # halfway (in the logarithm) between the smallest norm before the k-th and its own: the first met there
+        if n[k] >= 0.5 * min(n[:k]):
+            continue
+        rule = np.sqrt(n[k] * min(n[:k]))
+        for _ in range(60):
+            assert j.solveCoupledLinSysNS(A, b, rule, 0.0, 50)[1] == k
