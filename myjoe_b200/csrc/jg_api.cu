@@ -795,7 +795,10 @@ static int build(jg_case* h, const jg_mesh* mesh, const jg_params* q) {
       // per cell its line position and the number of its couplings off the line, per slice their last ELL row
       std::vector<int> line_pos(N, -1);
       std::vector<int> off_end(nslices);
-      for (int i = 0; i < off[L.nlines]; i++) line_pos[cv[i]] = i;
+      for (int i = 0; i < off[L.nlines]; i++) {
+        if (line_pos[cv[i]] >= 0) return set_err(JG_ERR_ARG, "cell %d is on two lines", cv[i]);
+        line_pos[cv[i]] = i;
+      }
       for (int sl = 0; sl < nslices; sl++) {
         int w = 0;
         for (int c = sl * SLICE; c < std::min(N, (sl + 1) * SLICE); c++) w = std::max(w, noff[c]);

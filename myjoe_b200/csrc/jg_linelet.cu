@@ -67,7 +67,15 @@ int build_lines(const jg_mesh& m, const std::vector<std::vector<int>>& wall_zone
   }
   off.assign(1, 0);
   cv.clear();
+  // a cell with several WALL faces is a source for each of them.  The reference grows a line from each;
+  // relaxed: one line only, since the LINE relaxation solves a cell's system once (the cell's couplings
+  // to two lines would be counted in both, and both would write its unknowns)
+  std::vector<char> headed(relaxed ? N : 0, 0);
   for (int s : src) {
+    if (relaxed) {
+      if (headed[s]) continue;
+      headed[s] = 1;
+    }
     const size_t first = cv.size();
     cv.push_back(s);
     for (;;) {

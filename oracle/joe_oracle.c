@@ -2034,7 +2034,8 @@ static int find_face(const jg_mesh *m, int a, int b) {
  * 0.5 |A_f| (1/V_cell + 1/V_nb) exceeds half the cell's largest neighbour
  * weight; two or more candidates (an isotropic region) or none end it.
  * With `relaxed` (the lines of the LINE relaxation, not the reference's),
- * every WALL zone's cells start lines, and a
+ * every WALL zone's cells start lines (one each, however many WALL faces the
+ * cell has: the reference starts one per WALL face), and a
  * line also goes on when several candidates pass but the strongest is more
  * than 1.1 times the next: so it crosses from a prism row into the hexahedron
  * above, whose other lower neighbour is the second prism of the quad. */
@@ -2058,10 +2059,14 @@ static void build_lines(jo_case *h, int relaxed, int *nlines_out, int **off_out,
   int cap = nsrc + 16, len = 0;
   int *cv = (int *)malloc(sizeof(int) * cap);
   int *off = (int *)malloc(sizeof(int) * (nsrc + 1));
+  unsigned char *headed = (unsigned char *)calloc(N ? N : 1, 1);
+  int l = 0;
   off[0] = 0;
-  for (int l = 0; l < nsrc; l++) {
+  for (int k = 0; k < nsrc; k++) {
+    if (relaxed && headed[src[k]]) continue;
+    headed[src[k]] = 1;
     if (len + 1 > cap) { cap *= 2; cv = (int *)realloc(cv, sizeof(int) * cap); }
-    cv[len++] = src[l];
+    cv[len++] = src[k];
     int index_cv = 0, add;
     do {
       int icv = cv[off[l] + index_cv];
@@ -2105,13 +2110,14 @@ static void build_lines(jo_case *h, int relaxed, int *nlines_out, int **off_out,
         index_cv++;
       }
     } while (add);
-    off[l + 1] = len;
+    off[++l] = len;
   }
-  *nlines_out = nsrc;
+  *nlines_out = l;
   *off_out = off;
   *cv_out = cv;
   free(src);
   free(check);
+  free(headed);
 }
 
 void jo_build_linelets(jo_case *h) {

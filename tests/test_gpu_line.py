@@ -119,3 +119,30 @@ def test_line_converged_sa_field_matches_oracle(precision):
     for a, b in zip(j.get_state(), o.get_state()):
         assert rel_l2(a, b) <= 1e-8
     assert rel_l2(j.get_scalars(), o.get_scalar()) <= 1e-8
+
+
+@pytest.mark.parametrize("renumber", [0, 3])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_line_solve_where_a_cell_has_two_wall_faces(precision, renumber):
+    """the cell is on one line: one sweep is the oracle's, and the sweeps converge to the system's solution"""
+    import scipy.sparse
+    import scipy.sparse.linalg
+    from myjoe_b200 import build, solver
+    from oracle.oracle import Oracle
+    from tests.test_lines import two_wall_face_case
+    build.build()
+    g, prm = two_wall_face_case(shuffle=True)
+    rng = np.random.default_rng(4)
+    A = rng.standard_normal((g.nbocv_v.shape[0], 5, 5))
+    A[g.nbocv_i[:-1]] += 40.0 * np.eye(5)
+    b = rng.standard_normal((g.ncv, 5))
+    j = solver.JoeGpu(g, prm, precision=precision, renumber=renumber)
+    o = Oracle(g, prm)
+    eps = np.finfo(np.float32).eps if precision else np.finfo(np.float64).eps
+    # rows of at most 7 blocks of 5 and a diagonal of about 40: a solve loses a few tens of roundings, and
+    # a sweep contracts the ones before it
+    for sweeps in (1, 4):
+        assert nrel(j.solveCoupledLinSysNS(A, b, 0, 0, sweeps)[0], o.solve(A, b, 0, 0, sweeps, 5)[0]) <= 200 * eps
+    M = scipy.sparse.bsr_matrix((A, g.nbocv_v, g.nbocv_i), shape=(5 * g.ncv, 5 * g.ncv)).tocsc()
+    want = scipy.sparse.linalg.spsolve(M, b.ravel())
+    assert nrel(j.solveCoupledLinSysNS(A, b, 0, 0, 60)[0], want) <= 200 * eps

@@ -10,6 +10,7 @@ stretched hexahedra and stop only where the cells turn isotropic."""
 import dataclasses
 
 import numpy as np
+import pytest
 
 from myjoe_b200 import case
 from oracle.oracle import Oracle
@@ -81,3 +82,36 @@ def test_rcm_lines_order_makes_each_line_consecutive():
         seg = pos[cv[off[l]:off[l + 1]]]
         assert np.all(np.diff(seg) == 1)
     assert (line_of >= 0).mean() > 0.6
+
+
+def two_wall_face_case(shuffle=False):
+    """Hexahedra growing away from a WALL that is two faces of one cell, on y- and z-: the cell has a
+    free neighbour along y and, when that one is taken, the next strongest along z, so that a line from
+    each of its WALL faces would have two cells or more."""
+    from myjoe_b200 import geometry, meshgen
+    x, z = 1.8 * np.arange(8.0), 1.3 * np.arange(5.0)
+    y = np.cumsum([0.0, 1.0, 1.1, 1.21, 1.33, 1.46])
+    X, Y = np.meshgrid(x, y, indexing="ij")
+
+    def zone(side, i, j, k):
+        here = (i == 3) & (j == 0) & (k == 0) & (side in ("jmin", "kmin"))
+        return np.where(here, "corner", "rest")
+    prm = dataclasses.replace(case.bump_case(4, 2, 2)[2], LINEAR_SOLVER_NS="LINE",
+                              bcs={"corner": case.BC("WALL"), "rest": case.BC("SYMMETRY")})
+    return geometry.build_cv_mesh(meshgen.structured_hex(X, Y, z, zone), seed=2, shuffle=shuffle), prm
+
+
+@pytest.mark.parametrize("shuffle", [False, True])
+def test_a_cell_with_two_wall_faces_heads_one_relaxed_line(shuffle):
+    from myjoe_b200 import solver
+    g, prm = two_wall_face_case(shuffle)
+    o = Oracle(g, prm)
+    off, cv = o.relax_lines()
+    assert len(off) == 2 and len(np.unique(cv)) == len(cv) >= 3
+    assert len(o.linelets()[0]) == 3   # the reference's rule: a line per WALL face
+    # the library's lines order the cells: each once
+    got = solver.renumber_cells(g, prm, solver.RENUMBER_RCM_LINES)
+    np.testing.assert_array_equal(np.sort(got), np.arange(g.ncv))
+    pos = np.empty(g.ncv, int)
+    pos[got] = np.arange(g.ncv)
+    assert np.all(np.diff(pos[cv]) == 1)
