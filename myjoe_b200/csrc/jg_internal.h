@@ -295,8 +295,10 @@ void launch_aos_to_soa5(int n, const double* aos, double* soa, cudaStream_t s);
 // LINE relaxation of the assembled system (block size bs, matrix precision of p): the
 // block-tridiagonal factors of every line, then `sweeps` line-Jacobi sweeps from x = 0;
 // the result is in st.x0 (odd sweeps) or st.x1 (even)
+// wait_tries: the limit of each wait of the substitutions for their copies
+constexpr int WAIT_TRIES = 1 << 20;
 void launch_line_relax(const Mesh& m, const Params& p, State& st, const Lines& L, int bs, int sweeps,
-                       cudaStream_t s);
+                       cudaStream_t s, int wait_tries = WAIT_TRIES);
 
 // one BiCGSTAB solve (jg_bicgstab.cu): vectors [5][N], the partial sums of the reductions (2,048
 // doubles), 16 doubles of device scalars, and the host's view of the iteration count (low half) and

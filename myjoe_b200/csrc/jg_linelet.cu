@@ -434,9 +434,9 @@ __device__ __forceinline__ void bulk_copy(void* dst, const void* p, unsigned len
 __device__ __forceinline__ void bar_expect(uint64_t* bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sh_addr(bar)), "r"(bytes) : "memory");
 }
-// false if the barrier's phase has not completed after a bounded number of tries
-__device__ __forceinline__ bool bar_wait(uint64_t* bar, unsigned parity) {
-  for (int i = 0; i < 1 << 20; i++) {
+// false if the barrier's phase has not completed after `tries` tries
+__device__ __forceinline__ bool bar_wait(uint64_t* bar, unsigned parity, int tries) {
+  for (int i = 0; i < tries; i++) {
     unsigned ok;
     asm volatile(
         "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
@@ -484,10 +484,13 @@ __device__ __forceinline__ void load_row(BT o[B], const BT* p) {
 // into shared memory and a step's instructions are its row loads, shuffles and multiply-adds: with
 // about one warp per scheduler it is the instructions of a step that cost.  2,048 lines of 20 to 80
 // cells, register double-buffering before -> now: 6x6 FP64 44 -> 39 us, FP32 36 -> 25; 7x7 FP32 32 -> 21.
-// The shuffles run on every lane; a group past the end of its line only skips the update.  A stage
-// that never completes (err gets 8) ends the pass, not the kernel's copies.
+// The shuffles run on every lane; a group past the end of its line only skips the update.  A wait
+// that runs out (tries) ends the warp's work with the steps of its stage, whose values are then
+// undefined: no further copies or steps; the warp waits for the copies it has in flight, within a
+// limit, sets flag 8 in err and returns.  (The vote on it stands after a stage's steps: between the
+// wait and the steps it costs 2-4% of the kernel.)
 template <typename BT, int B>
-__global__ void __launch_bounds__(32) k_lsolve(Mesh m, Lines L, BT* __restrict__ x, int* err) {
+__global__ void __launch_bounds__(32) k_lsolve(Mesh m, Lines L, BT* __restrict__ x, int* err, int tries) {
   static_assert(B <= LG, "a line's rows fit its lane group");
   using R = LineRing<BT, B>;
   constexpr int BB = B * B, K = R::LK, S = R::LS;
@@ -513,7 +516,11 @@ __global__ void __launch_bounds__(32) k_lsolve(Mesh m, Lines L, BT* __restrict__
   const BT* Lup = (const BT*)L.bup;
   BT* Lv = (BT*)L.bv;
   const int chunks = (nmax - 1 + K - 1) / K;  // steps 0 .. nmax - 2 of each pass
-  bool ok = true;
+  // the stages q .. asked - 1 are still in flight: wait for them, report, and the caller returns
+  auto give_up = [&](int q, int asked) {
+    for (; q < asked; q++) bar_wait(&bars[q % S], (q / S) & 1, WAIT_TRIES);
+    if (lane == 0) atomicOr(err, 8);
+  };
   // forward: v_0 = r_0, v_i = r_i - low_i v_{i-1}; step j is position j + 1.  Stage q % S holds the
   // q-th chunk asked for, forward chunks first
   auto ask_fwd = [&](int c) {
@@ -534,7 +541,7 @@ __global__ void __launch_bounds__(32) k_lsolve(Mesh m, Lines L, BT* __restrict__
   for (int c = 0; c < S - 1; c++) ask_fwd(c);
   BT v = has ? Lv[(size_t)p0 * B + rr] : BT(0);
   for (int c = 0; c < chunks; c++) {
-    ok = bar_wait(&bars[c % S], (c / S) & 1) && ok;
+    const bool ok = bar_wait(&bars[c % S], (c / S) & 1, tries);
     const int i0 = c * K + 1;
     const unsigned char* d = ring[c % S][g];
     const BT* lo = reinterpret_cast<const BT*>(d + shift16(Llow + (size_t)(p0 + i0) * BB)) + B * rr;
@@ -554,6 +561,7 @@ __global__ void __launch_bounds__(32) k_lsolve(Mesh m, Lines L, BT* __restrict__
       }
     }
     __syncwarp();
+    if (!__all_sync(0xffffffffu, ok)) return give_up(c, min(c + S - 1, chunks));
     ask_fwd(c + S - 1);
   }
   // the copy engine reads v back: the stores above first
@@ -596,7 +604,7 @@ __global__ void __launch_bounds__(32) k_lsolve(Mesh m, Lines L, BT* __restrict__
     int cell[K];
 #pragma unroll
     for (int t = 0; t < K; t++) cell[t] = hi - t >= 0 ? L.cv[p0 + hi - t] : 0;
-    ok = bar_wait(&bars[q0 % S], (q0 / S) & 1) && ok;
+    const bool ok = bar_wait(&bars[q0 % S], (q0 / S) & 1, tries);
     const unsigned char* d = ring[q0 % S][g];
     const BT* up = reinterpret_cast<const BT*>(d + shift16(Lup + (size_t)(p0 + l0 + 1) * BB)) + B * rr;
     const BT* iv = reinterpret_cast<const BT*>(d + R::BLK + shift16(Linv + (size_t)(p0 + l0) * BB)) + B * rr;
@@ -621,13 +629,13 @@ __global__ void __launch_bounds__(32) k_lsolve(Mesh m, Lines L, BT* __restrict__
       }
     }
     __syncwarp();
+    if (!__all_sync(0xffffffffu, ok)) return give_up(q0, chunks + min(c + S - 1, chunks));
     ask_bwd(c + S - 1);
   }
-  if (!ok && lane == 0) atomicOr(err, 8);
 }
 
 template <typename BT, int B>
-void line_relax(const Mesh& m, State& st, const Lines& L, int sweeps, cudaStream_t s) {
+void line_relax(const Mesh& m, State& st, const Lines& L, int sweeps, cudaStream_t s, int wait_tries) {
   const int lb = (L.nlines + LW - 1) / LW;
   if (L.nlines) k_lfactor<BT, B><<<lb, 32 * LW, 0, s>>>(m, st, L);
   for (int it = 0; it < sweeps; it++) {
@@ -638,20 +646,19 @@ void line_relax(const Mesh& m, State& st, const Lines& L, int sweeps, cudaStream
     // (a pass's early blocks take the SMs of the substitutions, which are a chain of latencies)
     k_sweep<BT, B, SWEEP_LINE, 2, sizeof(BT) == 4 ? 1600 / (B * SLICE) : 1><<<m.nslices, B * SLICE, 0, s>>>(
         m, st, xin, xout, it == 0, -1, nullptr, L.line_pos, L.noff, L.off_end, (BT*)L.bv);
-    if (L.nlines) k_lsolve<BT, B><<<(L.nlines + LPW - 1) / LPW, 32, 0, s>>>(m, L, xout, st.err);
+    if (L.nlines) k_lsolve<BT, B><<<(L.nlines + LPW - 1) / LPW, 32, 0, s>>>(m, L, xout, st.err, wait_tries);
   }
 }
 
 }  // namespace
 
 void launch_line_relax(const Mesh& m, const Params& p, State& st, const Lines& L, int bs, int sweeps,
-                       cudaStream_t s) {
+                       cudaStream_t s, int wait_tries) {
   sweeps = sweeps < 1 ? 1 : sweeps;
-  switch (bs) {
-    case 5: p.fp32 ? line_relax<float, 5>(m, st, L, sweeps, s) : line_relax<double, 5>(m, st, L, sweeps, s); break;
-    case 6: p.fp32 ? line_relax<float, 6>(m, st, L, sweeps, s) : line_relax<double, 6>(m, st, L, sweeps, s); break;
-    default: p.fp32 ? line_relax<float, 7>(m, st, L, sweeps, s) : line_relax<double, 7>(m, st, L, sweeps, s); break;
-  }
+  auto run = bs == 5   ? (p.fp32 ? line_relax<float, 5> : line_relax<double, 5>)
+             : bs == 6 ? (p.fp32 ? line_relax<float, 6> : line_relax<double, 6>)
+                       : (p.fp32 ? line_relax<float, 7> : line_relax<double, 7>);
+  run(m, st, L, sweeps, s, wait_tries);
 }
 
 }  // namespace jg
