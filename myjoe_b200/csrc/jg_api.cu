@@ -1191,6 +1191,13 @@ static int pinned(jg_case* h, size_t bytes, void** out) {
   return JG_OK;
 }
 
+// what a handle's error flags (not zero) mean
+static int flags_error(int e) {
+  if (e & 2) return set_err(JG_ERR_ARG, "unrecognised boundary condition");
+  if (e & 8) return set_err(JG_ERR_CUDA, "line substitutions: an asynchronous copy did not complete");
+  return set_err(JG_ERR_STATE, "non-physical state (flags %d): negative density/pressure or NaN residual", e);
+}
+
 // Reads (and clears) the error flags; with nres > 0 also copies nres doubles from the device
 // array dres to res_out, in the same synchronisation (the copy is made whatever the flags say).
 static int check_err_flags(jg_case* h, bool all_cases = false, const double* dres = nullptr, size_t nres = 0,
@@ -1214,9 +1221,7 @@ static int check_err_flags(jg_case* h, bool all_cases = false, const double* dre
   }
   if (e) {
     CK(cudaMemsetAsync(h->st.err, 0, sizeof(int), h->stream));
-    if (e & 2) return set_err(JG_ERR_ARG, "unrecognised boundary condition");
-    if (e & 8) return set_err(JG_ERR_CUDA, "line substitutions: an asynchronous copy did not complete");
-    return set_err(JG_ERR_STATE, "non-physical state (flags %d): negative density/pressure or NaN residual", e);
+    return flags_error(e);
   }
   return JG_OK;
 }
@@ -1532,6 +1537,18 @@ int jg_solve_lin_sys(jg_case_t* h, double* dq, const double* A, const double* rh
   }
   CKL();
   RC(download_rows(h, h->st.dq, dq, h->rn.cell_old, N, 5));
+  if (h->hp.lin_solver == JG_LS_LINE) {
+    // of the flags only the solve's own: a state's stay for the call that reads them
+    int e = 0;
+    CK(cudaMemcpyAsync(&e, h->st.err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    if (e & 8) {
+      e &= ~8;
+      CK(cudaMemcpyAsync(h->st.err, &e, sizeof(int), cudaMemcpyHostToDevice, h->stream));
+      CK(cudaStreamSynchronize(h->stream));
+      return flags_error(8);
+    }
+  }
   if (iters) *iters = it;
   return JG_OK;
 }
@@ -1808,9 +1825,7 @@ int jg_step_host(jg_case_t* h, double* rho, double* rhou, double* rhoE, int nste
     const double* o = (const double*)hp;
     if (nres) memcpy(resid, o + 2, nres * sizeof(double));
     const int e = (int)o[0] | (int)o[1];
-    if (e & 2) return set_err(JG_ERR_ARG, "unrecognised boundary condition");
-    if (e) return set_err(JG_ERR_STATE, "non-physical state (flags %d): negative density/pressure or NaN residual", e);
-    return JG_OK;
+    return e ? flags_error(e) : JG_OK;
   }
   RC(stage_state_in(h, rho, rhou, rhoE));
   RC(prime_enqueue(h));

@@ -111,3 +111,11 @@ def _run(stand_in, *args):
 def test_a_step_whose_wait_runs_out_is_a_cuda_error(stand_in, model, precision):
     out = _run(stand_in, "step", model, str(precision))
     assert "code -2" in out and "asynchronous copy" in out and "done" in out, out
+
+
+@pytest.mark.parametrize("call", ["step_host", "solve"])
+@pytest.mark.parametrize("model,precision", [("none", 0), ("none", 1)])
+def test_every_call_reports_it(stand_in, call, model, precision):
+    """not as a diverged state (step_host), nor as success (one linear solve)"""
+    out = _run(stand_in, call, model, str(precision))
+    assert "code -2" in out and "asynchronous copy" in out and "done" in out, out
