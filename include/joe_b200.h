@@ -337,7 +337,8 @@ int jg_batch_set_active(jg_case_t *h, int case_id, int active);
  * per cell sums them; the same kernels for every FL) and a Jacobian
  * kernel (one thread per cell, the face matrices formed row by row) on two
  * streams.  Second: the kernel of the 5x5 Jacobi sweep (0: a block per 32-cell
- * slice, a thread per block row, the default; 1: a thread per cell).
+ * slice, a thread per block row; 1: a thread per cell; the default is 0, and 1
+ * for mixed handles of the sizes where its blocks fill the GPU).
  * jg_autotune times each candidate on the handle's own mesh (trials launches,
  * CUDA events) and keeps the fastest; ms[10] (may be NULL) gets the face loop
  * time per launch: fused 1, 2, 4 lanes (ms[0..2]), fused JG_FLUX_CL1_3BLK

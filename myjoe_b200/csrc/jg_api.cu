@@ -593,6 +593,7 @@ static int build(jg_case* h, const jg_mesh* mesh, const jg_params* q) {
     for (int c = 0; c <= ncolors; c++) m.color_slice_off[c] = coff[c];
   }
   m.ncv = N; m.nfa = nfa; m.nfa_b = nfa_b; m.nzones = mesh->nzones; m.nslices = nslices; m.ell_rows = rows;
+  if (bs == 5) h->p.relax_variant = jacobi_variant(m, h->p);  // jg_set_launch_config changes it
   RC(upload(h, &m.x_cv, mesh->x_cv, 3 * (size_t)N));
   RC(upload(h, &m.vol, mesh->cv_volume, (size_t)N));
   RC(upload(h, &m.x_fa, mesh->x_fa, 3 * (size_t)nfa));

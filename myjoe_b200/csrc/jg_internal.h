@@ -217,6 +217,7 @@ constexpr int RCHUNK = 256;
 void launch_resid_cases(State& st, const int* case_off, const int* rblk_off, const int* rblk_case, int nrblk,
                         int ncases, int hist_from_ctrl, cudaStream_t s);
 void launch_jacobi(const Mesh& m, const Params& p, State& st, int sweeps, cudaStream_t s);
+int jacobi_variant(const Mesh& m, const Params& p);  // the sweep kernel (Params::relax_variant) a mesh starts with
 // multicolour Gauss-Seidel: result in st.x0
 void launch_sgs(const Mesh& m, const Params& p, State& st, int sweeps, cudaStream_t s);
 void launch_dq_from_x(const Mesh& m, const Params& p, State& st, const void* x, cudaStream_t s);

@@ -1095,12 +1095,23 @@ void launch_face_sensors(const Mesh& m, const Params& p, State& st, cudaStream_t
 void launch_grad_coupled(const Mesh& m, const Params& p, State& st, cudaStream_t s) {
   launch_grad_k(m, p, st, p.second_order, 1, p.limiter, p.limiter, 0, s);
 }
+// FP64 rows run a slice at a time at every size.  An FP32 sweep streams better a cell per thread where
+// that kernel's resident blocks are well filled: the second wave of a grid just above one is nearly
+// empty, and far below one its few long threads do not cover their latency.  w: the grid in waves.  us
+// per sweep, slice / cell kernel, six columns a row (8 x 120 x nx): w 0.59 31.0 / 34.4, 0.74 37.2 / 37.4,
+// 0.80 40.5 / 39.1, 0.99 48.9 / 43.4, 1.01 50.1 / 55.7, 1.22 59.3 / 62.8, 1.35 66.6 / 66.2, 1.48 73.1 /
+// 68.7, 2.02 97.3 / 92.6, 6.6 322 / 250.  Rows of four (one layer of cells) gain earlier: w 0.53 21.4 /
+// 19.9, 0.99 42.8 / 34.3, 1.06 45.1 / 47.3, 1.22 52.1 / 49.3
+int jacobi_variant(const Mesh& m, const Params& p) {
+  if (!p.fp32) return 0;
+  static const int fit = resident_blocks(k_jacobi<float>, TB);
+  const double w = (double)grid_for(m.ncv, TB) / fit;
+  const bool narrow = 2L * m.ell_rows <= 9L * m.nslices;  // four and a half columns a row or fewer
+  return w <= 1.0 ? w >= (narrow ? 0.5 : 0.77) : w >= (narrow ? 1.2 : 1.35);
+}
 // both sweep kernels do the same arithmetic in the same order (bit-identical results)
 void launch_jacobi(const Mesh& m, const Params& p, State& st, int sweeps, cudaStream_t s) {
-  // FP32 rows stream better a cell per thread once the matrix is well above L2 (us per ten sweeps, slice
-  // kernel / this one: 100k cells 109 / 129, 250k 344 / 326, 700k 938 / 867); the bits are the same
-  const bool cells = p.relax_variant == 1 || (p.fp32 && m.nslices > 5000);
-  if (!cells) {
+  if (p.relax_variant == 0) {
     if (p.fp32) sweep_jacobi<float, 5>(m, st, sweeps, s);
     else sweep_jacobi<double, 5>(m, st, sweeps, s);
     return;

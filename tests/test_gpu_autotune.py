@@ -86,3 +86,37 @@ def test_batch_bitwise_under_a_shared_shape():
         for x, y in zip(b.get_case_state(k), st):
             np.testing.assert_array_equal(x, y)
     b.close()
+
+
+def _sweep_kernels(j, g):
+    """names of the kernels of one Jacobi solve"""
+    from torch.profiler import ProfilerActivity, profile
+    rng = np.random.default_rng(3)
+    A = rng.standard_normal((g.nbocv_v.shape[0], 5, 5))
+    A[g.nbocv_i[:-1]] += 40.0 * np.eye(5)
+    b = rng.standard_normal((g.ncv, 5))
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        x, _ = j.solveCoupledLinSysNS(A, b, 0.0, 0.0, 3)
+    names = {e.key for e in prof.key_averages()}
+    return x, {k for k in ("k_sweep", "k_jacobi") if any(k in n for n in names)}
+
+
+# an FP32 sweep a cell per thread where its grid fills the GPU: 9k cells no, 224k in one layer yes, 350k
+# (a wave and a fifth of it) no, 500k (a wave and two thirds) yes; FP64 never
+@pytest.mark.parametrize("dims,precision,default", [((96, 48, 2), 1, 0), ((560, 400, 1), 1, 1), ((560, 400, 1), 0, 0),
+                                                    ((500, 350, 2), 1, 0), ((714, 350, 2), 1, 1)])
+def test_the_sweep_kernel_asked_for_runs(dims, precision, default):
+    _, g, prm = case.bump_case(*dims)
+    prm = dataclasses.replace(prm, LINEAR_SOLVER_NS="JACOBI", LS_MAX_ITER=3)
+    j = solver.JoeGpu(g, prm, precision=precision)
+    assert j.launch_config() == (36, default)
+    out = []
+    for variant in (None, 0, 1):
+        if variant is not None:
+            j.set_launch_config(36, variant)
+        x, ran = _sweep_kernels(j, g)
+        assert ran == {("k_sweep", "k_jacobi")[default if variant is None else variant]}
+        out.append(x)
+    np.testing.assert_array_equal(out[1], out[0])
+    np.testing.assert_array_equal(out[2], out[0])
+    j.close()
