@@ -342,9 +342,10 @@ int jg_batch_set_active(jg_case_t *h, int case_id, int active);
  * jg_autotune times each candidate on the handle's own mesh (trials launches,
  * CUDA events) and keeps the fastest; ms[10] (may be NULL) gets the face loop
  * time per launch: fused 1, 2, 4 lanes (ms[0..2]), fused JG_FLUX_CL1_3BLK
- * (ms[5]), split FL = 1, 2, 4, 8 (ms[6..9]); and the sweep time for kernels 0,
- * 1 (ms[3..4]).  A handle with a lagged Jacobian (jac_lag > 1) runs split
- * shapes only.  The sweep kernels give bit-identical results; the face-loop
+ * (ms[5]), split (ms[6..9], one shape and one time; the one chosen is
+ * JG_FLUX_SPLIT + 4); and the sweep time for kernels 0, 1 (ms[3..4]).  A
+ * handle with a lagged Jacobian (jac_lag > 1) runs the split shape only.  The
+ * sweep kernels give bit-identical results; the face-loop
  * shapes change the order of each cell's diagonal-block and residual sums
  * (rounding-level differences).  Handles without a turbulence model; others
  * keep their single shape.  A batch handle tunes for all its cases. */

@@ -2174,13 +2174,13 @@ extern "C" int jg_autotune(jg_case_t* h, int trials, int* flux_cl, int* relax_va
     State st = h->st;
     st.jac_lag = 1;
     // ms[0..2]: fused, 1, 2, 4 lanes per cell; ms[5]: fused, one lane with three blocks per SM;
-    // ms[6..9]: split (one shape under four names).  A lagged handle runs split.
-    const int cls[8] = {1, 2, 4, JG_FLUX_CL1_3BLK, JG_FLUX_SPLIT + 1, JG_FLUX_SPLIT + 2, JG_FLUX_SPLIT + 4,
-                        JG_FLUX_SPLIT + 8};
-    const int slot[8] = {0, 1, 2, 5, 6, 7, 8, 9};
+    // ms[6..9]: split, one shape under four names, timed and chosen as the default's.  A lagged handle
+    // runs split.
+    const int cls[5] = {1, 2, 4, JG_FLUX_CL1_3BLK, JG_FLUX_SPLIT + 4};
+    const int slot[5] = {0, 1, 2, 5, 8};
     float best = 1e30f;
     int best_cl = h->p.flux_cl, best_v = h->p.relax_variant;
-    for (int i = 0; i < 8; i++) {
+    for (int i = 0; i < 5; i++) {
       if (h->st.jac_lag > 1 && cls[i] < JG_FLUX_SPLIT) {
         if (ms) ms[slot[i]] = 0.0f;
         continue;
@@ -2196,6 +2196,7 @@ extern "C" int jg_autotune(jg_case_t* h, int trials, int* flux_cl, int* relax_va
       if (ms) ms[slot[i]] = t_ms / trials;
       if (t_ms < best) { best = t_ms; best_cl = cls[i]; }
     }
+    if (ms) ms[6] = ms[7] = ms[9] = ms[8];
     p.flux_cl = best_cl;
     best = 1e30f;
     for (int v = 0; v < 2; v++) {

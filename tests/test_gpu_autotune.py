@@ -120,3 +120,14 @@ def test_the_sweep_kernel_asked_for_runs(dims, precision, default):
     np.testing.assert_array_equal(out[1], out[0])
     np.testing.assert_array_equal(out[2], out[0])
     j.close()
+
+
+def test_autotune_times_the_split_shape_once():
+    """its four names are one shape: one time, and the name chosen is the default's, not the noise's"""
+    g, prm = _plate()
+    j = solver.JoeGpu(g, prm, jac_lag=4)   # a lagged handle has the split shape only
+    j.set_state(*case.perturbed_state(g.x_cv, prm, 0.02))
+    for _ in range(4):
+        cl, _, ms = j.autotune(2)
+        assert cl == 36 and len({ms["flux_cl%d" % (32 + k)] for k in (1, 2, 4, 8)}) == 1
+    j.close()
