@@ -881,12 +881,12 @@ static size_t footprint(const jg_mesh* mesh, const jg_params* q, const std::vect
       3 * N * d, N * d, 3 * nfa * d, 3 * nfa * d, 2 * nfa * i, 4 * N * d, 8 * nfa * d, std::max<size_t>(4 * (nfa - nfa_b), 1) * d,
       (N + 1) * i, (size_t)fi[N] * sizeof(Slot),
       (N + 1) * i, nbs * i, 3 * nbs * d, (N + 1) * i, std::max<size_t>(nbslot, 1) * i, 3 * nfa_b * d,
-      nfa_b * i, nz * sizeof(DevZone), (nslices + 1) * i, rows * SLICE * i, rows * SLICE, N,
+      nfa_b * i, nz * sizeof(DevZone), (nslices + 1) * i, std::max<size_t>(rows * SLICE * i, 1), std::max<size_t>(rows * SLICE, 1), N,
       // state
       5 * N * d, 8 * N * d, 8 * nfa_b * d, nfa * d, nfa * d, GS * N * d,
       (q->mu_ref > 0.0 && q->second_order && !q->visc_limiter && q->limiter && bs == 5) ? GS * N * d : 0,
       GHS * N * d, bs == 5 ? (q->mu_ref > 0.0 ? 12 : 8) * nfa * d : 0, N * d, bs * N * d, bs * N * d,
-      b2 * N * e, b2 * N * e, bs > 5 && e == 4 ? b2 * N * d : 0, rows * b2 * SLICE * e, bs * N * e, bs * N * e, bs * N * d,
+      b2 * N * e, b2 * N * e, bs > 5 && e == 4 ? b2 * N * d : 0, std::max<size_t>(rows * b2 * SLICE * e, 1), bs * N * e, bs * N * e, bs * N * d,
       (5 * (size_t)grid_for((int)N, 16) + 5 * (size_t)grid_for((int)N, 256) + 16) * d, 16 * d, 4 * i,
       bs * 64 * d, 2 * i, N * i, 1 * i, 1,
       2 * i, ((N + RCHUNK - 1) / RCHUNK) * i, bs * ((N + RCHUNK - 1) / RCHUNK) * d,

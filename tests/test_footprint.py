@@ -1,0 +1,33 @@
+"""Device memory a case needs (jg_case_footprint, the serving engine's admission rule): host only."""
+import dataclasses
+
+import pytest
+
+from myjoe_b200 import case, solver
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims", [(1, 1, 1), (2, 1, 1), (3, 2, 1), (16, 8, 2)])
+@pytest.mark.parametrize("model", ["NONE", "SA"])
+def test_a_handle_holds_its_footprint(model, dims):
+    """from the meshes whose matrix is smaller than their centres on, and the records are right: a step gives
+    the oracle's residual"""
+    import numpy as np
+    from oracle.oracle import Oracle
+    sa = model == "SA"
+    _, g, prm = (case.sa_bump_case if sa else case.bump_case)(*dims)
+    prm = dataclasses.replace(prm, LINEAR_SOLVER_NS="JACOBI")
+    st = case.perturbed_state(g.x_cv, prm, 0.02)
+    j = solver.JoeGpu(g, prm, precision=1)
+    j.set_state(*st)
+    assert j.device_bytes() == solver.case_footprint(g, prm, 1)
+    if not sa:
+        o = Oracle(g, prm)
+        o.set_state(*st)
+        o.calc_state()
+        o.calc_dt()
+        rho, rhou, rhoE, _ = o.calc_rhs(False)
+        got = j.calcRhs(False)[:3]
+        # sums of at most six face fluxes of the order of p u, rho u, rho E u
+        for a, b, s in zip(got, (rho, rhou, rhoE), o.array("flux_scale").max(0)[[0, 1, 4]]):
+            assert np.abs(a - np.reshape(b, a.shape)).max() <= 1e-11 * max(s, 1e-300)
