@@ -175,6 +175,19 @@ static int upload(jg_case* h, const T** dst, const T* src, size_t count) {
   return JG_OK;
 }
 
+// gives an array of `bytes` back (after the work enqueued on it)
+static int dfree(jg_case* h, void* p, size_t bytes) {
+  h->allocs.erase(std::find(h->allocs.begin(), h->allocs.end(), p));
+  h->bytes -= alloc_round(bytes);
+  if (h->async_alloc) {
+    CK(cudaFreeAsync(p, h->stream));
+  } else {
+    CK(cudaStreamSynchronize(h->stream));
+    CK(cudaFree(p));
+  }
+  return JG_OK;
+}
+
 // a device array of the handle -> the caller's host array, rows in the caller's order
 static int download_rows(jg_case* h, const double* dev, double* host, const std::vector<int>& perm, size_t n,
                          size_t w, size_t nblk = 1) {
@@ -594,9 +607,7 @@ static int build(jg_case* h, const jg_mesh* mesh, const jg_params* q) {
   }
   m.ncv = N; m.nfa = nfa; m.nfa_b = nfa_b; m.nzones = mesh->nzones; m.nslices = nslices; m.ell_rows = rows;
   if (bs == 5) h->p.relax_variant = jacobi_variant(m, h->p);  // jg_set_launch_config changes it
-  RC(upload(h, &m.x_cv, mesh->x_cv, 3 * (size_t)N));
   RC(upload(h, &m.vol, mesh->cv_volume, (size_t)N));
-  RC(upload(h, &m.x_fa, mesh->x_fa, 3 * (size_t)nfa));
   RC(upload(h, &m.fa_n, mesh->fa_normal, 3 * (size_t)nfa));
   RC(upload(h, &m.cvofa, mesh->cvofa, 2 * (size_t)nfa));
   {
@@ -624,8 +635,6 @@ static int build(jg_case* h, const jg_mesh* mesh, const jg_params* q) {
   RC(upload(h, &m.color, color.data(), color.size()));
   m.ncolors = ncolors;
   m.color_proper = proper;
-  launch_geo(m, (double*)m.xv, (double*)m.fa_u, (double*)m.fa_s, h->stream);
-  CKL();
   // device state
   State& st = h->st;
   memset(&st, 0, sizeof(st));
@@ -662,6 +671,21 @@ static int build(jg_case* h, const jg_mesh* mesh, const jg_params* q) {
   RC(dmalloc_bytes(h, &st.Dinv, bs * bs * (size_t)N * h->eltsz));
   if (bs > 5 && h->eltsz == 4) RC(dmalloc(h, &st.dfull, bs * bs * (size_t)N));
   RC(dmalloc_bytes(h, &st.O, h->ell_elems * h->eltsz));
+  {
+    // the centres live in the geometry records only: the caller's arrays stand in the matrix (its padding
+    // is zero again after) while the records are formed, or in an array of their own where it is smaller
+    const size_t nx = 3 * (size_t)N, bytes = (nx + 3 * (size_t)nfa) * sizeof(double);
+    const bool fits = h->ell_elems * h->eltsz >= bytes;
+    void* at = st.O;
+    if (!fits) RC(dmalloc_bytes(h, &at, bytes));
+    double* x = (double*)at;
+    CK(cudaMemcpyAsync(x, mesh->x_cv, nx * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+    CK(cudaMemcpyAsync(x + nx, mesh->x_fa, bytes - nx * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+    launch_geo(m, x, x + nx, (double*)m.xv, (double*)m.fa_u, (double*)m.fa_s, h->stream);
+    CKL();
+    if (fits) CK(cudaMemsetAsync(at, 0, bytes, h->stream));
+    else RC(dfree(h, at, bytes));
+  }
   RC(dmalloc_bytes(h, &st.x0, bs * (size_t)N * h->eltsz));
   RC(dmalloc_bytes(h, &st.x1, bs * (size_t)N * h->eltsz));
   RC(dmalloc(h, &st.dq, bs * (size_t)N));
@@ -878,7 +902,7 @@ static size_t footprint(const jg_mesh* mesh, const jg_params* q, const std::vect
   const size_t nz = std::max(1, mesh->nzones);
   const size_t a[] = {
       // mesh
-      3 * N * d, N * d, 3 * nfa * d, 3 * nfa * d, 2 * nfa * i, 4 * N * d, 8 * nfa * d, std::max<size_t>(4 * (nfa - nfa_b), 1) * d,
+      N * d, 3 * nfa * d, 2 * nfa * i, 4 * N * d, 8 * nfa * d, std::max<size_t>(4 * (nfa - nfa_b), 1) * d,
       (N + 1) * i, (size_t)fi[N] * sizeof(Slot),
       (N + 1) * i, nbs * i, 3 * nbs * d, (N + 1) * i, std::max<size_t>(nbslot, 1) * i, 3 * nfa_b * d,
       nfa_b * i, nz * sizeof(DevZone), (nslices + 1) * i, std::max<size_t>(rows * SLICE * i, 1), std::max<size_t>(rows * SLICE, 1), N,

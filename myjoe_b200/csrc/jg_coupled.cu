@@ -53,13 +53,13 @@ __global__ void __launch_bounds__(256) k_wall_dist(Mesh m, Turb t, int c0, int c
   const int nwall = w1 - w0;
   double x[3] = {0.0, 0.0, 0.0};
   if (c < c1)
-    for (int i = 0; i < 3; i++) x[i] = m.x_cv[3 * c + i];
+    for (int i = 0; i < 3; i++) x[i] = m.xv[(size_t)4 * c + i];
   double minD = 1.0e20;
   int save = 0;
   for (int k0 = 0; k0 < nwall; k0 += 256) {
     int k = k0 + threadIdx.x;
     if (k < nwall)
-      for (int i = 0; i < 3; i++) sx[threadIdx.x][i] = m.x_fa[3 * t.wall_f[w0 + k] + i];
+      for (int i = 0; i < 3; i++) sx[threadIdx.x][i] = m.fa_u[(size_t)8 * t.wall_f[w0 + k] + 4 + i];
     __syncthreads();
     int n = min(256, nwall - k0);
     for (int j = 0; j < n; j++) {
@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(256) k_wall_dist(Mesh m, Turb t, int c0, int c
   int f = t.wall_f[w0 + save];
   double n[3], sh[3], nmag;
   unit_normal_c(m, f, n, nmag);
-  for (int i = 0; i < 3; i++) sh[i] = m.x_fa[3 * f + i] - x[i];
+  for (int i = 0; i < 3; i++) sh[i] = m.fa_u[(size_t)8 * f + 4 + i] - x[i];
   double sMag2 = dot3(sh, sh);
   double dNorm2 = dot3(sh, n) * dot3(sh, n);
   double dTang2 = sMag2 - dNorm2;
@@ -148,7 +148,7 @@ __global__ void k_grad_phi(Mesh m, Params p, Turb t) {
           Slot sl = m.slots[k];
           if (sl.nb < 0) continue;
           double r0[3];
-          for (int j = 0; j < 3; j++) r0[j] = m.x_fa[3 * sl.f + j] - m.x_cv[3 * c + j];
+          cell_to_face(m, c, sl.f, r0);
           double phifa = pc + dot3(r0, g);
           double dm = phifa - pc;
           double dp = ((phifa - pc) >= 0.0) ? pmax - pc : pmin - pc;
@@ -218,10 +218,8 @@ __global__ void k_turb_face(Mesh m, State st, Turb t) {
   if (f >= m.nfa_b) {
     int c0 = m.cvofa[2 * f], c1 = m.cvofa[2 * f + 1];
     double d0[3], d1[3];
-    for (int i = 0; i < 3; i++) {
-      d0[i] = m.x_fa[3 * f + i] - m.x_cv[3 * c0 + i];
-      d1[i] = m.x_fa[3 * f + i] - m.x_cv[3 * c1 + i];
-    }
+    cell_to_face(m, c0, f, d0);
+    cell_to_face(m, c1, f, d1);
     double w0 = sqrt(dot3(d0, d0)), w1 = sqrt(dot3(d1, d1));
     double rho_fa = (w1 * st.q[5 * c0] + w0 * st.q[5 * c1]) / (w0 + w1);
     if (!sst) {
@@ -857,10 +855,8 @@ __global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb
         double kine_fa = 0.0;
         if (SST) {
           double d0[3], d1[3];
-          for (int i = 0; i < 3; i++) {
-            d0[i] = m.x_fa[3 * f + i] - m.x_cv[3 * c0 + i];
-            d1[i] = m.x_fa[3 * f + i] - m.x_cv[3 * c1 + i];
-          }
+          cell_to_face(m, c0, f, d0);
+          cell_to_face(m, c1, f, d1);
           double w0 = sqrt(dot3(d0, d0)), w1 = sqrt(dot3(d1, d1));
           kine_fa = (w1 * v0.k + w0 * v1.k) / (w0 + w1);
         }
@@ -915,7 +911,7 @@ __global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb
           for (int q = 0; q < NS; q++) vb.sc[q] = Bs.sc[q];
           vb.k = Bs.k;
           double sV[3];
-          for (int i = 0; i < 3; i++) sV[i] = m.x_fa[3 * f + i] - m.x_cv[3 * c + i];
+          cell_to_face(m, c, f, sV);
           double smag = fabs(dot3(sV, nV));
           VFC<NS> vf;
           visc_flux_c<NS>(F, vf, vb, vb, st.mul_fa[f], st.mut_fa[f], st.lam_fa[f], p.PrTurb, Bs.k, vb.u, dfa, one,
@@ -948,7 +944,7 @@ __global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb
           vb.gs[q] = v0.gs[q];
         }
         double sV[3];
-        for (int i = 0; i < 3; i++) sV[i] = m.x_fa[3 * f + i] - m.x_cv[3 * c + i];
+        cell_to_face(m, c, f, sV);
         double smag = fabs(dot3(sV, nV));
         VFC<NS> vf;
         visc_flux_c<NS>(F, vf, v0, vb, st.mul_fa[f], 0.0, st.lam_fa[f], p.PrTurb, 0.0, vb.u, dfa, dterm, area, nV,
@@ -979,7 +975,7 @@ __global__ void __launch_bounds__(128) k_flux_c(Mesh m, Params p, State st, Turb
         }
         vb.k = Bs.k;
         double sV[3];
-        for (int i = 0; i < 3; i++) sV[i] = m.x_fa[3 * f + i] - m.x_cv[3 * c + i];
+        cell_to_face(m, c, f, sV);
         double smag = sqrt(dot3(sV, sV));
         for (int i = 0; i < 3; i++) sV[i] /= smag;
         double alpha = dot3(nV, sV);

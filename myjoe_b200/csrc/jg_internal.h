@@ -35,13 +35,12 @@ struct Slot {
 struct Mesh {
   int ncv, nfa, nfa_b, nzones;
   int nslices;
-  const double* x_cv;      // [N][3]
   const double* vol;       // [N]
-  const double* x_fa;      // [nfa][3]
   const double* fa_n;      // [nfa][3] area-weighted normal
   // static geometry records, formed once per mesh (k_cell_geo, k_face_geo) with the expressions the
   // face loop used to evaluate per face and laid out for its 32-byte loads: xv[N][4] centre and
-  // volume; fa_u[nfa][8] the unit normal, the area, the face centre and a pad; fa_s[nfa - nfa_b][4] the unit
+  // volume; fa_u[nfa][8] the unit normal, the area, the face centre and a pad (the only copies of the
+  // centres); fa_s[nfa - nfa_b][4] the unit
   // vector from cvofa[f][0]'s centre to cvofa[f][1]'s and its length (sVec, smag) of internal faces
   const double* xv;
   const double* fa_u;
@@ -199,7 +198,8 @@ void launch_grad(const Mesh& m, const Params& p, State& st, cudaStream_t s);
 void launch_flux(const Mesh& m, const Params& p, State& st, int implicit, int for_step, cudaStream_t s);
 void launch_flux_fused(const Mesh& m, const Params& p, State& st, int for_step, cudaStream_t s);
 void launch_face_sensors(const Mesh& m, const Params& p, State& st, cudaStream_t s);
-void launch_geo(const Mesh& m, double* xv, double* fa_u, double* fa_s, cudaStream_t s);
+void launch_geo(const Mesh& m, const double* x_cv, const double* x_fa, double* xv, double* fa_u, double* fa_s,
+                cudaStream_t s);
 // jg_step_host's upload (pack + state + history base) and download (unpack + flags + residuals)
 void launch_state_in(const Mesh& m, const Params& p, State& st, const double* rho, const double* rhou,
                      const double* rhoE, const int* perm, cudaStream_t s);

@@ -405,7 +405,8 @@ __device__ void grad_sdwls(const Mesh& m, const Params& p, const State& st, int 
   Sdwls M[4];
   for (int q = 0; q < 4; q++)
     for (int k = 0; k < 6; k++) M[q].sw[k] = 0.0;
-  double den[4] = {0.0, 0.0, 0.0, 0.0};
+  double den[4] = {0.0, 0.0, 0.0, 0.0}, xc[4];
+  ld4(xc, &m.xv[(size_t)4 * c]);
   for (int j = 0; j < 9; j++) gu[j] = 0.0;
   for (int j = 0; j < 3; j++) gr[j] = gpr[j] = gh[j] = 0.0;
   for (int pass = 0; pass < 2; pass++) {
@@ -415,8 +416,9 @@ __device__ void grad_sdwls(const Mesh& m, const Params& p, const State& st, int 
       const int nb = m.nb_v[k];
       const double* pn = &st.prim[8 * nb];
       const double v[6] = {pn[0], pn[1], pn[2], st.q[5 * nb], pn[3], pn[5]};
-      double dx[3];
-      for (int i = 0; i < 3; i++) dx[i] = m.x_cv[3 * nb + i] - m.x_cv[3 * c + i];
+      double xn[4], dx[3];
+      ld4(xn, &m.xv[(size_t)4 * nb]);
+      for (int i = 0; i < 3; i++) dx[i] = xn[i] - xc[i];
       sdwls_visit(pass, dx, vc, v, e, M, den, gu, gr, gpr, gh);
     }
     for (int k = m.bf_i[c]; k < m.bf_i[c + 1]; k++) {
@@ -424,7 +426,7 @@ __device__ void grad_sdwls(const Mesh& m, const Params& p, const State& st, int 
       const double* b = &st.bfa[8 * f];
       const double v[6] = {b[1], b[2], b[3], b[0], b[4], b[6]};
       double dx[3];
-      for (int i = 0; i < 3; i++) dx[i] = m.x_fa[3 * f + i] - m.x_cv[3 * c + i];
+      cell_to_face(m, c, f, dx);
       sdwls_visit(pass, dx, vc, v, e, M, den, gu, gr, gpr, gh);
     }
   }
@@ -501,10 +503,8 @@ __global__ void __launch_bounds__(128, MINB) k_grad(Mesh m, Params p, State st, 
       if (s.nb < 0) continue;
       const int f = s.f, c0 = m.cvofa[2 * f], c1 = m.cvofa[2 * f + 1];
       double d0[3], d1[3];
-      for (int j = 0; j < 3; j++) {
-        d0[j] = m.x_fa[3 * f + j] - m.x_cv[3 * c0 + j];
-        d1[j] = m.x_fa[3 * f + j] - m.x_cv[3 * c1 + j];
-      }
+      cell_to_face(m, c0, f, d0);
+      cell_to_face(m, c1, f, d1);
       const double w0 = sqrt(dot3(d0, d0)), w1 = sqrt(dot3(d1, d1));
       const double* p0 = &st.prim[8 * c0];
       const double* p1 = &st.prim[8 * c1];
@@ -994,7 +994,7 @@ constexpr int TB = 128;
 
 // static face geometry, once per mesh: the unit normal and area of every face; for internal
 // faces the unit vector between the cell centres and its length
-__global__ void k_face_geo(Mesh m, double* fa_u, double* fa_s) {
+__global__ void k_face_geo(Mesh m, const double* x_cv, const double* x_fa, double* fa_u, double* fa_s) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= m.nfa) return;
   const double n[3] = {m.fa_n[3 * f], m.fa_n[3 * f + 1], m.fa_n[3 * f + 2]};
@@ -1002,29 +1002,30 @@ __global__ void k_face_geo(Mesh m, double* fa_u, double* fa_s) {
   double* u = &fa_u[8 * (size_t)f];
   for (int i = 0; i < 3; i++) {
     u[i] = n[i] / area;
-    u[4 + i] = m.x_fa[3 * f + i];
+    u[4 + i] = x_fa[3 * (size_t)f + i];
   }
   u[3] = area;
   u[7] = 0.0;
   if (f >= m.nfa_b) {
     const int c0 = m.cvofa[2 * f], c1 = m.cvofa[2 * f + 1];
     double sV[3];
-    for (int i = 0; i < 3; i++) sV[i] = m.x_cv[3 * c1 + i] - m.x_cv[3 * c0 + i];
+    for (int i = 0; i < 3; i++) sV[i] = x_cv[3 * (size_t)c1 + i] - x_cv[3 * (size_t)c0 + i];
     const double smag = sqrt(dot3(sV, sV));
     double* o = &fa_s[4 * (f - m.nfa_b)];
     for (int i = 0; i < 3; i++) o[i] = sV[i] / smag;
     o[3] = smag;
   }
 }
-__global__ void k_cell_geo(Mesh m, double* xv) {
+__global__ void k_cell_geo(Mesh m, const double* x_cv, double* xv) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.ncv) return;
-  for (int i = 0; i < 3; i++) xv[4 * (size_t)c + i] = m.x_cv[3 * (size_t)c + i];
+  for (int i = 0; i < 3; i++) xv[4 * (size_t)c + i] = x_cv[3 * (size_t)c + i];
   xv[4 * (size_t)c + 3] = m.vol[c];
 }
-void launch_geo(const Mesh& m, double* xv, double* fa_u, double* fa_s, cudaStream_t s) {
-  k_cell_geo<<<grid_for(m.ncv, TB), TB, 0, s>>>(m, xv);
-  if (m.nfa > 0) k_face_geo<<<grid_for(m.nfa, TB), TB, 0, s>>>(m, fa_u, fa_s);
+void launch_geo(const Mesh& m, const double* x_cv, const double* x_fa, double* xv, double* fa_u, double* fa_s,
+                cudaStream_t s) {
+  k_cell_geo<<<grid_for(m.ncv, TB), TB, 0, s>>>(m, x_cv, xv);
+  if (m.nfa > 0) k_face_geo<<<grid_for(m.nfa, TB), TB, 0, s>>>(m, x_cv, x_fa, fa_u, fa_s);
 }
 
 void launch_state(const Mesh& m, const Params& p, State& st, cudaStream_t s) {

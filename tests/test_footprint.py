@@ -6,6 +6,15 @@ import pytest
 from myjoe_b200 import case, solver
 
 
+@pytest.mark.parametrize("precision,limit", [(0, 3100), (1, 2320)])
+def test_centres_are_held_once(precision, limit):
+    """8,192 hexahedra: 288 bytes a cell of state, ~370 of gradients and face fluxes, 25 blocks of 25,
+    and cell and face centres in their records only (24 bytes a cell and a face each)"""
+    _, g, prm = case.bump_case(64, 32, 4)
+    prm = dataclasses.replace(prm, LINEAR_SOLVER_NS="SGS")
+    assert solver.case_footprint(g, prm, precision) / g.ncv <= limit
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("dims", [(1, 1, 1), (2, 1, 1), (3, 2, 1), (16, 8, 2)])
 @pytest.mark.parametrize("model", ["NONE", "SA"])
