@@ -459,6 +459,12 @@ static int color_cells(const jg_mesh* mesh, std::vector<uint8_t>& color, std::ve
   return ncolors;
 }
 
+// the coupled HLLC blocks are inverted by a kernel of their own, from the FP64 diagonal: a copy of it
+// beside FP32 blocks.  The AUSM family inverts where it forms them
+static bool inverts_apart(int bs, const jg_params& q) {
+  return bs > 5 && q.precision == JG_PREC_MIXED && q.flux != JG_FLUX_AUSMDV && q.flux != JG_FLUX_HAENEL;
+}
+
 static int build(jg_case* h, const jg_mesh* mesh, const jg_params* q) {
   const int N = mesh->ncv, nfa = mesh->nfa, nfa_b = mesh->nfa_b;
   if (!h->stream) CK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
@@ -669,7 +675,7 @@ static int build(jg_case* h, const jg_mesh* mesh, const jg_params* q) {
   RC(dmalloc(h, &st.b, bs * (size_t)N));
   RC(dmalloc_bytes(h, &st.D, bs * bs * (size_t)N * h->eltsz));
   RC(dmalloc_bytes(h, &st.Dinv, bs * bs * (size_t)N * h->eltsz));
-  if (bs > 5 && h->eltsz == 4) RC(dmalloc(h, &st.dfull, bs * bs * (size_t)N));
+  if (inverts_apart(bs, *q)) RC(dmalloc(h, &st.dfull, bs * bs * (size_t)N));
   RC(dmalloc_bytes(h, &st.O, h->ell_elems * h->eltsz));
   {
     // the centres live in the geometry records only: the caller's arrays stand in the matrix (its padding
@@ -910,7 +916,7 @@ static size_t footprint(const jg_mesh* mesh, const jg_params* q, const std::vect
       5 * N * d, 8 * N * d, 8 * nfa_b * d, nfa * d, nfa * d, GS * N * d,
       (q->mu_ref > 0.0 && q->second_order && !q->visc_limiter && q->limiter && bs == 5) ? GS * N * d : 0,
       GHS * N * d, bs == 5 ? (q->mu_ref > 0.0 ? 12 : 8) * nfa * d : 0, N * d, bs * N * d, bs * N * d,
-      b2 * N * e, b2 * N * e, bs > 5 && e == 4 ? b2 * N * d : 0, std::max<size_t>(rows * b2 * SLICE * e, 1), bs * N * e, bs * N * e, bs * N * d,
+      b2 * N * e, b2 * N * e, inverts_apart((int)bs, *q) ? b2 * N * d : 0, std::max<size_t>(rows * b2 * SLICE * e, 1), bs * N * e, bs * N * e, bs * N * d,
       (5 * (size_t)grid_for((int)N, 16) + 5 * (size_t)grid_for((int)N, 256) + 16) * d, 16 * d, 4 * i,
       bs * 64 * d, 2 * i, N * i, 1 * i, 1,
       2 * i, ((N + RCHUNK - 1) / RCHUNK) * i, bs * ((N + RCHUNK - 1) / RCHUNK) * d,

@@ -15,6 +15,16 @@ def test_centres_are_held_once(precision, limit):
     assert solver.case_footprint(g, prm, precision) / g.ncv <= limit
 
 
+@pytest.mark.parametrize("flux", ["AUSMDV", "HAENEL"])
+@pytest.mark.parametrize("model,b", [("SA", 6), ("SST", 7)])
+def test_only_hllc_keeps_the_fp64_diagonal_of_a_mixed_handle(model, b, flux):
+    """its blocks are inverted by a kernel of their own; the AUSM family inverts where it forms them"""
+    _, g, prm = (case.sa_bump_case if model == "SA" else case.sst_bump_case)(32, 16, 2)
+    prm = dataclasses.replace(prm, LINEAR_SOLVER_NS="SGS", SHOCK_FIX_TYPE="NONE")
+    hllc, other = (solver.case_footprint(g, dataclasses.replace(prm, SPACE_INTEGRATION=f), 1) for f in ("HLLC", flux))
+    assert hllc - other == 8 * b * b * g.ncv
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("dims", [(1, 1, 1), (2, 1, 1), (3, 2, 1), (16, 8, 2)])
 @pytest.mark.parametrize("model", ["NONE", "SA"])
