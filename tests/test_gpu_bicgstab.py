@@ -96,3 +96,15 @@ def test_reported_count_is_that_of_the_stopping_iteration():
         rule = np.sqrt(n[k] * min(n[:k]))
         for _ in range(60):
             assert j.solveCoupledLinSysNS(A, b, rule, 0.0, 50)[1] == k
+
+
+def test_iterates_above_the_reductions_grid_cap():
+    """270,000 unknowns: the dot products' 1,024 blocks stride over them and fill the partial sums"""
+    g, prm, A, b = _system((300, 180, 1), 0, np.random.default_rng(8))
+    j = solver.JoeGpu(g, prm)
+    for iterations in (1, 2, 3):
+        x, it = j.solveCoupledLinSysNS(A, b, -1.0, -1.0, iterations - 1)
+        assert it == iterations
+        want = _bicgstab(g, A, b, iterations)
+        # as on the small systems; the sums are seven times longer than the largest of them
+        assert np.abs(x - want).max() <= 1e-11 * 10 ** (iterations - 1) * np.abs(want).max()

@@ -55,3 +55,23 @@ def test_gradients_cost_a_few_state_reads():
             t.append(time.perf_counter() - a)
         return 1e3 * float(np.median(t))
     assert ms(j.gradients) <= 15.0 * ms(j.get_state)
+
+
+def test_gradients_match_the_oracle_on_several_waves():
+    """144,000 cells: the least-squares kernel compiled for four resident blocks per SM"""
+    _, g, prm = case.bump_case(360, 200, 2)
+    prm = dataclasses.replace(prm, MU_REF=1.0e-3)
+    st = case.perturbed_state(g.x_cv, prm, 0.05)
+    o = Oracle(g, prm)
+    o.set_state(*st)
+    o.calc_state()
+    o.calc_dt()
+    o.calc_rhs(False)
+    j = solver.JoeGpu(g, prm)
+    j.set_state(*st)
+    got = j.calcGrad()
+    scale = {"grad_u": np.abs(st[1] / st[0][:, None]).max(), "grad_rho": st[0].max(), "grad_p": 1.0e5,
+             "grad_enthalpy": 4.0e5}
+    lsq = max(np.abs(g.nbocv_lsg_coeff).max(), np.abs(g.boundary_fa_lsg_coeff).max())
+    for k in NAMES:
+        assert np.abs(got[k].ravel() - o.array(k).ravel()).max() <= 1e-12 * lsq * scale[k], k

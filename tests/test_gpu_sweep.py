@@ -89,3 +89,66 @@ def test_sweep_kernels_agree_bitwise_around_one_wave(nx, ny):
         j.close()
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+# FP32 rows: 160 threads of 80 registers, five blocks per SM, so 740 slices (23,680 cells) are one wave of the
+# whole-row kernel; above it runs capped at 64 registers
+@pytest.mark.parametrize("nx,ny", [(148, 128), (197, 120), (197, 124), (350, 230)])
+def test_fp32_sweep_kernels_agree_bitwise_around_one_wave(nx, ny):
+    g, prm = _mesh(nx, ny, 1)
+    prm = dataclasses.replace(prm, LINEAR_SOLVER_NS="JACOBI", LS_MAX_ITER=4)
+    A, b = _system(g, np.random.default_rng(2))
+    out = []
+    for variant in (0, 1):
+        j = solver.JoeGpu(g, prm, precision=1)
+        j.set_launch_config(36, variant)
+        out.append(j.solveCoupledLinSysNS(A, b, 0.0, 0.0, 4)[0])
+        j.close()
+    np.testing.assert_array_equal(*out)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("nx,ny,renumber", [(197, 120, 0), (250, 200, 0)])
+def test_sgs_matches_plain_numpy_around_one_wave(nx, ny, renumber, precision):
+    g, prm = _mesh(nx, ny, 1)
+    prm = dataclasses.replace(prm, LINEAR_SOLVER_NS="SGS", LS_MAX_ITER=3)
+    A, b = _system(g, np.random.default_rng(7))
+    j = solver.JoeGpu(g, prm, precision=precision, renumber=renumber)
+    x, _ = j.solveCoupledLinSysNS(A, b, 0.0, 0.0, 3)
+    want = _relax(g, A, b, 3, _colors(g))
+    tol = 500.0 * (np.finfo(np.float32).eps if precision else np.finfo(np.float64).eps)   # as above
+    assert np.abs(x - want).max() <= tol * np.abs(want).max()
+
+
+# coupled blocks: one wave of the whole-row kernel is at most 592 slices of 6x6 FP64 (four blocks per SM),
+# less of 7x7, more of FP32; 36k cells are 1,125 slices
+@pytest.mark.parametrize("name", ["JACOBI", "SGS"])
+@pytest.mark.parametrize("model", ["SA", "SST"])
+def test_coupled_steps_match_the_oracle_above_one_wave(model, name):
+    from oracle.oracle import OracleSA
+    sa = model == "SA"
+    _, g, prm = (case.sa_bump_case if sa else case.sst_bump_case)(180, 100, 2, stretch=1.03)
+    prm = dataclasses.replace(prm, LINEAR_SOLVER_NS=name, LS_MAX_ITER=4, CFL=1.0)
+    st = case.perturbed_state(g.x_cv, prm, 0.0)
+    phi = np.full(g.ncv, prm.NUSA_INITIAL) if sa else np.tile([prm.KINE_INITIAL, prm.OMEGA_INITIAL], (g.ncv, 1))
+    o = OracleSA(g, prm)
+    o.set_state(*st)
+    o.set_scalar(phi)
+    o.calc_state()
+    o.step(1)
+    out = []
+    for precision in (0, 1):
+        j = solver.JoeGpu(g, prm, precision=precision)
+        j.set_state(*st)
+        j.set_scalars(phi)
+        j.runBackwardEuler(1)
+        out.append([*j.get_state(), j.get_scalars()])
+        j.close()
+    for a, m, b, s in zip(out[0], out[1], [*o.get_state(), o.get_scalar()], [*st, phi]):
+        a, m, b, s = (np.asarray(x, float).reshape(g.ncv, -1) for x in (a, m, b, s))
+        groups = [slice(0, 3)] if a.shape[1] == 3 else [slice(k, k + 1) for k in range(a.shape[1])]
+        for k in groups:   # the momentum as one vector, each scalar by itself
+            assert np.abs(a[:, k] - b[:, k]).max() <= 1e-10 * np.abs(b[:, k]).max()   # as the steps of test_gpu_sa
+            # FP32 blocks: the update to single precision, of which the conditioning of the blocks takes at
+            # most a factor 1e3
+            assert np.abs(m[:, k] - a[:, k]).max() <= 1e-4 * np.abs(a[:, k] - s[:, k]).max()
