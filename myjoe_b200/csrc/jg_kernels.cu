@@ -434,8 +434,8 @@ __device__ void grad_sdwls(const Mesh& m, const Params& p, const State& st, int 
 
 // SCHEME: the gradient scheme (JG_GRAD_*) as a template parameter, so that each
 // scheme's kernel holds only its own registers.  MINB: resident blocks per SM.  A thread's rows and
-// records arrive by gathers whose latency other warps cover: 137 registers leave three blocks,
-// capped at 128 (24 bytes of spills) four.  The cap pays once the grid is several waves
+// records arrive by gathers whose latency other warps cover: 152 registers leave three blocks,
+// capped at 128 (24 bytes of spills) four
 template <int SCHEME, int MINB>
 __global__ void __launch_bounds__(128, MINB) k_grad(Mesh m, Params p, State st, int do_euler, int do_visc, int visc_lim_u, int visc_lim_h,
                        int separate_guv) {
@@ -1064,13 +1064,17 @@ void launch_dt(const Mesh& m, const Params& p, State& st, int use_ctrl, double c
 static void launch_grad_k(const Mesh& m, const Params& p, State& st, int do_euler, int do_visc, int lim_u, int lim_h,
                           int separate, cudaStream_t s) {
   const int g = grid_for(m.ncv, TB);
-  // least squares above seven blocks per SM (148): four resident blocks.  us, three -> four: 64 blocks
-  // 11.9 -> 12.2, 384 (viscous) 16.4 -> 17.4, 784 (viscous) 37 -> 39, 2,344 88 -> 72
+  // least squares compiled for three or for four resident blocks (444 or 592 on the GPU): a wave of four
+  // takes 7 to 10% longer, so four where that makes a wave less.  us, three / four, blocks: 444 12.6 / 13.8,
+  // 460 21.2 / 15.7, 592 23.0 / 16.8, 620 22.4 / 23.9, 888 29.9 / 32.5, 960 41.5 / 34.4, 1,184 46.3 / 38.6,
+  // 1,300 46.8 / 49.3, 1,500 60.3 / 52.4, 2,344 88.8 / 73.0, 3,500 120.9 / 105.0
+  static const int fit3 = resident_blocks(k_grad<JG_GRAD_LSQ, 1>, TB), fit4 = resident_blocks(k_grad<JG_GRAD_LSQ, 4>, TB);
+  const bool four = (g + fit4 - 1) / fit4 < (g + fit3 - 1) / fit3;
   if (p.grad_scheme == JG_GRAD_GREENGAUSS)
     k_grad<JG_GRAD_GREENGAUSS, 1><<<g, TB, 0, s>>>(m, p, st, do_euler, do_visc, lim_u, lim_h, separate);
   else if (p.grad_scheme == JG_GRAD_SDWLS)
     k_grad<JG_GRAD_SDWLS, 1><<<g, TB, 0, s>>>(m, p, st, do_euler, do_visc, lim_u, lim_h, separate);
-  else if (g > 7 * 148)
+  else if (four)
     k_grad<JG_GRAD_LSQ, 4><<<g, TB, 0, s>>>(m, p, st, do_euler, do_visc, lim_u, lim_h, separate);
   else
     k_grad<JG_GRAD_LSQ, 1><<<g, TB, 0, s>>>(m, p, st, do_euler, do_visc, lim_u, lim_h, separate);

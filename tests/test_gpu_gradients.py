@@ -57,9 +57,11 @@ def test_gradients_cost_a_few_state_reads():
     assert ms(j.gradients) <= 15.0 * ms(j.get_state)
 
 
-def test_gradients_match_the_oracle_on_several_waves():
-    """144,000 cells: the least-squares kernel compiled for four resident blocks per SM"""
-    _, g, prm = case.bump_case(360, 200, 2)
+# 148 SMs: up to 444 blocks of 128 cells are a wave of three resident blocks per SM, up to 592 of four
+@pytest.mark.parametrize("dims", [(200, 142, 2), (200, 143, 2), (200, 189, 2), (200, 190, 2), (360, 200, 2)])
+def test_gradients_match_the_oracle_where_the_kernel_changes(dims):
+    """the least-squares kernel compiled for three or for four resident blocks per SM"""
+    _, g, prm = case.bump_case(*dims)
     prm = dataclasses.replace(prm, MU_REF=1.0e-3)
     st = case.perturbed_state(g.x_cv, prm, 0.05)
     o = Oracle(g, prm)
