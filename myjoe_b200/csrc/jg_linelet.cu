@@ -641,10 +641,13 @@ void line_relax(const Mesh& m, State& st, const Lines& L, int sweeps, cudaStream
   for (int it = 0; it < sweeps; it++) {
     BT* xin = (BT*)((it % 2 == 0) ? st.x1 : st.x0);
     BT* xout = (BT*)((it % 2 == 0) ? st.x0 : st.x1);
-    // two columns at a time: most line cells have three or four couplings off their line.  The passes
+    // two columns at a time: most line cells have three or four couplings off their line.  FP32 resident
+    // blocks by measurement (us a pass): 5x5 8 / 9 / 10 8.6 / 8.6 / 7.5 (32 registers, 8 bytes of spills,
+    // and one wave of the 49k-cell plate), 6x6 6 / 8 23.2 / 21.1, 7x7 5 / 6 / 7 21.7 / 21.1 / 22.0.  The passes
     // and substitutions are plain launches: as programmatic dependents they measured 4-5% slower
     // (a pass's early blocks take the SMs of the substitutions, which are a chain of latencies)
-    k_sweep<BT, B, SWEEP_LINE, 2, sizeof(BT) == 4 ? 1600 / (B * SLICE) : 1><<<m.nslices, B * SLICE, 0, s>>>(
+    constexpr int blocks = sizeof(BT) == 8 ? 1 : B == 5 ? 10 : B == 6 ? 8 : 6;
+    k_sweep<BT, B, SWEEP_LINE, 2, blocks><<<m.nslices, B * SLICE, 0, s>>>(
         m, st, xin, xout, it == 0, -1, nullptr, L.line_pos, L.noff, L.off_end, (BT*)L.bv);
     if (L.nlines) k_lsolve<BT, B><<<(L.nlines + LPW - 1) / LPW, 32, 0, s>>>(m, L, xout, st.err, wait_tries);
   }
