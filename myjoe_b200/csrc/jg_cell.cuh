@@ -14,19 +14,7 @@ namespace jg {
 // an L1 prefetch of the cache line holding p (a hint: no registers held, no wait)
 __device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
-// the face loop's reads of a neighbour cell c, prefetched a face ahead: its state, primitives,
-// centre, gradients (and the viscous gradients)
-__device__ __forceinline__ void prefetch_cell(const State& st, const Mesh& m, int c, bool visc) {
-  prefetch_l1(&st.prim[(size_t)8 * c]);
-  prefetch_l1(&m.xv[(size_t)4 * c]);
-  prefetch_l1(&st.gu[(size_t)GS * c]);
-  if (visc) {
-    prefetch_l1(&st.guv[(size_t)GS * c]);
-    prefetch_l1(&st.gh[(size_t)GHS * c]);
-  }
-}
-
-// the Jacobian kernel's reads of a neighbour cell c: its state and primitives (and the viscous
+// the Jacobian kernel's reads of a neighbour cell c, prefetched a face ahead: its state and primitives (and the viscous
 // gradient the viscous matrices' stress needs)
 __device__ __forceinline__ void prefetch_cell_jac(const State& st, int c, bool visc) {
   prefetch_l1(&st.prim[(size_t)8 * c]);
