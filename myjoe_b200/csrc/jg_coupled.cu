@@ -143,12 +143,14 @@ __global__ void k_grad_phi(Mesh m, Params p, Turb t) {
     if (p.limiter) {
       double alfa = 1.0;
       if ((pmax - pmin) > 1.0e-12) {
-        double e2 = sq(fmax(p.eps * fabs(pc), 1.0e-8));
+        double e2 = sq(fmax(p.eps * fabs(pc), 1.0e-8)), xc[4];
+        ld4(xc, &m.xv[(size_t)4 * c]);
         for (int k = m.slot_i[c]; k < m.slot_i[c + 1]; k++) {
           Slot sl = m.slots[k];
           if (sl.nb < 0) continue;
-          double r0[3];
-          cell_to_face(m, c, sl.f, r0);
+          double xf[4], r0[3];
+          ld4(xf, &m.fa_u[(size_t)8 * sl.f + 4]);
+          for (int j = 0; j < 3; j++) r0[j] = xf[j] - xc[j];
           double phifa = pc + dot3(r0, g);
           double dm = phifa - pc;
           double dp = ((phifa - pc) >= 0.0) ? pmax - pc : pmin - pc;
