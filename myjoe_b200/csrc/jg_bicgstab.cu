@@ -10,7 +10,8 @@
 // iterations a step, the call with its state copies: 1,180 -> 612 us a step).
 //
 // The matrix products take a slice of 32 block rows per block, a warp per row, like the relaxation
-// passes (jg_sweep.cuh), their matrix rows requested while the vector update before them drains;
+// passes (jg_sweep.cuh), the diagonal block's row requested while the vector update before them drains
+// and the other blocks' two columns at a time;
 // the vector updates form their preconditioned vector in the same pass; the residual's product
 // subtracts from the right-hand side and takes the maximum norm on the way.  Reductions keep the
 // order of a grid of at most 1,024 blocks with a tree in each and over them.

@@ -5,7 +5,7 @@
 //    reconstruction, the Riemann flux and the viscous flux once; a thread per cell
 //    then sums its faces' fluxes.  Bound by the latency of the gathers and of the
 //    FP64 chains, so the work is cut into the most threads with the fewest registers
-//    (80 inviscid, 104 viscous): a thread per cell and four slots evaluated every
+//    (80 inviscid, 106 viscous): a thread per cell and four slots evaluated every
 //    internal face twice.  300k cells HLLC 169 -> 84 + 38 us, the 49k-cell viscous Roe
 //    plate 46 -> 24 + 10 us.
 //  * k_jac: the Jacobian blocks, which the reference forms at the cell-centre

@@ -15,9 +15,10 @@
 //    the next pass's blocks start while this one drains and have everything but x in registers
 //    when it ends.  x therefore goes through L2 only (__ldcg): an L1 line read by an earlier pass
 //    may not be seen by a later one that started before the boundary.
-// Measured, 10 sweeps, the loop over one column at a time before -> now: 8k cells FP64 Jacobi 61 ->
-// 35 us, 50k 84 -> 82, 250k 576 -> 535, 700k 1485 -> 1405 (5.8 -> 6.2 TB/s of matrix); FP32 8k 49 ->
-// 23; FP32 SGS 250k 299 -> 264 (20 passes -> 11 besides).
+// Measured, us per solve of 10 sweeps, a kernel taking one column at a time by plain launches -> this one
+// (two-layer bumps in colour order): FP64 Jacobi 8k cells 70 -> 29, 50k 84 -> 86, 250k 567 -> 528, 700k
+// 1454 -> 1376 (6.3 TB/s of matrix); FP32 Gauss-Seidel, two colours and so 11 passes instead of 20: 8k
+// 104 -> 25, 50k 111 -> 45, 250k 467 -> 266, 700k 1239 -> 696.
 //
 // Every sum keeps its order (k within a column, column by column), so the results are bit for bit
 // those of the thread-per-cell kernel (k_jacobi).
@@ -143,18 +144,18 @@ int resident_blocks(void (*kernel)(P...), int block) {
 
 // One pass.  A grid that fits the GPU in one wave takes the widest chunk of columns (the shortest
 // dependent chain); a larger FP64 grid lives on resident blocks instead, so it takes three columns
-// while those blocks fit one wave and one column with all 2,048 threads of an SM above.  FP32 rows
-// are half as wide in registers and take the whole row at any size (packed above one wave).  Us per solve (10 sweeps; FP64
-// Jacobi 8k / 35k / 50k / 250k / 700k cells): six columns 35 / 82 / 117 / 754 / 2012, three 37 / 55 /
-// 94 / 563 / 1487, one 43 / 76 / 82 / 535 / 1405; FP32 SGS 8k / 50k / 250k / 700k: six 25 / 41 / 242 /
-// 634, three 35 / 49 / 272 / 693, one 47 / 64 / 291 / 704.
+// while those blocks fit one wave and one column with up to 1,920 threads of an SM above.  FP32 rows
+// are half as wide in registers and take the whole row at any size, above one wave capped at the
+// registers of 960 threads per SM (left to itself the compiler takes 80 a thread).  us per solve of 10
+// sweeps, two-layer bumps in colour order (the 8k cells in four layers), 8k / 35k / 50k / 250k / 700k
+// cells.  FP64 Jacobi: six columns 29 / 74 / 100 / 633 / 1722, three 41 / 55 / 98 / 545 / 1430, one 49 /
+// 78 / 86 / 528 / 1376.  FP32 Gauss-Seidel: six 25 / 37 / 61 / 324 / 873, six capped 29 / 39 / 45 / 266 /
+// 696, three 35 / 41 / 51 / 281 / 711, one 57 / 55 / 70 / 297 / 719.
 template <typename BT, int B, int KIND>
 void launch_sweep(const Mesh& m, const State& st, int grid, const BT* xin, BT* xout, bool first, int color,
                   const int* slices, bool after_pass, cudaStream_t s) {
   constexpr int T = B * SLICE;
   auto wide = k_sweep<BT, B, KIND, SWEEP_COLS, 1>;
-  // FP32 above one wave: registers for 960 threads per SM (left to itself the compiler takes 80 a thread:
-  // 250k cells SGS 320 us a solve, capped 264; below one wave the uncapped kernel is 3% faster)
   auto packed = k_sweep<BT, B, KIND, SWEEP_COLS, sizeof(BT) == 4 ? 960 / T : 1>;
   auto mid = k_sweep<BT, B, KIND, 3, 1280 / T>;
   auto narrow = k_sweep<BT, B, KIND, 1, 1920 / T>;
