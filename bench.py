@@ -185,7 +185,7 @@ CONVERGE_WORKLOAD = ("burst of seeded channel-bump cases (hex, 2 cell layers; ce
 
 
 HBM_WORKLOAD = ("channel bump 1400x700x2 hex (1,960,000 cells), HLLC, second order, far field, JACOBI x10, "
-                "cells grouped by Gauss-Seidel colour in RCM order; the working set (~4 GB FP64) is far above L2")
+                "cells grouped by Gauss-Seidel colour in RCM order; the working set (~6 GB FP64) is far above L2")
 
 
 def build_hbm_case():
@@ -446,7 +446,7 @@ def main():
     e2e = world * n * args.steps / e2e_s
 
     # like for like with the reference arm: the same case with the GPU's BiCGSTAB x10 (the
-    # reference's LINEAR_SOLVER_NS_TRESHOLDS MAX_ITER=10), FP64, host-driven iterations
+    # reference's LINEAR_SOLVER_NS_TRESHOLDS MAX_ITER=10), FP64, iterations enqueued by the host
     jb = solver.JoeGpu(g, dataclasses.replace(prm, LINEAR_SOLVER_NS="BCGSTAB", LS_MAX_ITER=SWEEPS), precision=0)
     jb.set_state(*st0)
     jb.runBackwardEuler(max(args.warmup, 3))
@@ -459,7 +459,7 @@ def main():
     jb.close()
     bicgstab = {"value": g.ncv * nb / bcg_s, "unit": "cell-iters/s", "steps": nb,
                 "linear_solver": "BCGSTAB MAX_ITER=%d (the reference arm's solver), FP64" % SWEEPS,
-                "timing": "wall clock around synchronised host-driven steps"}
+                "timing": "wall clock around the synchronised call"}
 
     conv = converge_leg(conv_cases, args) if conv_cases else None
     hbm = None
@@ -488,8 +488,10 @@ def main():
     split = tuned_cl >= 32
     face_name = ("face loop: k_face_flux + k_res (residual) beside k_jac (Jacobian blocks) on a second stream"
                  if split else "k_flux (fused face loop + Jacobian assembly)")
+    sweep_name = ("k_jacobi (block point-relaxation sweep, a thread per cell)" if tuned_sweep else
+                  "k_sweep (block point-relaxation pass, a warp per block row of 32 cells)")
     if solve_avg >= face_avg:
-        dom = {"kernel": "k_jacobi (block point-relaxation sweep)", "bound": "hbm", "achieved": sweep_gbs,
+        dom = {"kernel": sweep_name, "bound": "hbm", "achieved": sweep_gbs,
                "peak": peak, "unit": "GB/s", "frac": sweep_gbs / peak, "traffic": None,
                "bytes_per_cell": sweep_b, "launch_ms": sweep_avg}
         other = {"kernel": face_name, "achieved": face_gbs, "frac": face_gbs / peak,
@@ -498,7 +500,7 @@ def main():
         dom = {"kernel": face_name, "bound": "hbm", "achieved": face_gbs,
                "peak": peak, "unit": "GB/s", "frac": face_gbs / peak, "traffic": None,
                "bytes_per_cell": face_b, "launch_ms": face_avg}
-        other = {"kernel": "k_jacobi (block point-relaxation sweep)", "achieved": sweep_gbs, "frac": sweep_gbs / peak,
+        other = {"kernel": sweep_name, "achieved": sweep_gbs, "frac": sweep_gbs / peak,
                  "bytes_per_cell": sweep_b, "launch_ms": sweep_avg}
     dom["launch_ms_source"] = ("CUDA events inside the step graph, averaged over a second pass of the same "
                                "steps (the timed steps run without the event nodes)")
@@ -507,11 +509,11 @@ def main():
     if os.path.exists(prof_path):
         with open(prof_path) as f:
             tr = json.load(f)
-        key = "k_jacobi" if dom["kernel"].startswith("k_jacobi") else "face_loop"
+        key = dom["kernel"].split()[0] if dom["kernel"].startswith(("k_sweep", "k_jacobi")) else "face_loop"
         if key in tr and args.precision in tr[key]:
             entry = tr[key][args.precision]
             if key == "face_loop":  # per launch shape
-                entry = entry.get(str(tuned_cl))
+                entry = entry.get("split" if split else str(tuned_cl))
             if entry:
                 dom["traffic"] = entry["bytes_per_cell"] * n
                 dom["traffic_source"] = entry["source"]
